@@ -1145,7 +1145,7 @@ static void fill_image_args(ImageArgs& a, const SlothGridDesc* g, const void* gr
 }
 
 struct ImageWs {
-    unsigned *hist, *keys, *perm, *skeys;
+    unsigned *hist, *keys, *perm, *offs;
     void* ckpt;
     int* nsteps;
     unsigned* bound;    // acceleration bound of the forward (float bits), in the header's second half
@@ -1159,7 +1159,7 @@ static ImageWs carve(void* ws, const SlothImageParams* p, long long n) {
     w.hist = reinterpret_cast<unsigned*>(base + kHeaderBytes);
     w.keys = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes);
     w.perm = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes + a);
-    w.skeys = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes + 2 * a);
+    w.offs = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes + 2 * a);
     char* c = base + workspace_bytes(n);
     w.ckpt = c;
     w.nsteps = reinterpret_cast<int*>(c + align256((size_t)(image_n_seg(p) + 1) * 48u * (size_t)(n > 0 ? n : 1)));
@@ -1198,14 +1198,13 @@ static int image_forward_impl(const SlothGridDesc* g, const void* grid, const Sl
     if (e != cudaSuccess) return cuda_status(e);
     if (n == 0) return SLOTH_OK;
     ImageWs w = carve(ws, p, n);
-    // One thread per ray in bucket order, with no tile sort: buckets of one
-    // transverse entry cell each (for grids of up to 513 points across the
-    // probing axis) keep a warp's rays in few cells, so that its cell loads
-    // and gradient flushes share addresses.
-    const int bbits = kMaxBucketBits;
-    if ((e = cudaMemsetAsync(w.hist, 0, (size_t)4 << bbits, s)) != cudaSuccess) return cuda_status(e);
-    rc = launch_prepass<typename P::R>(g, p->probing_axis, rays, n, bbits, w.keys, w.hist, w.perm, w.skeys, sms, s,
-                                       true);
+    // One thread per ray in bucket order: buckets of few rays keep a warp's
+    // rays in few cells, so that its cell loads and gradient flushes share
+    // addresses.
+    const int bbits = bucket_bits_for(n);
+    if ((e = cudaMemsetAsync(w.hist, 0, hist_bytes(bbits), s)) != cudaSuccess) return cuda_status(e);
+    rc = launch_prepass<typename P::R>(g, p->probing_axis, rays, n, bbits, w.keys, w.hist, w.perm, w.offs, nullptr,
+                                       sms, s);
     if (rc) return rc;
     ImageArgs a;
     fill_image_args(a, g, grid, p, rays, n, w.perm, w.ckpt, w.nsteps);

@@ -23,7 +23,7 @@
 // tiles run in the same kernels as the others' (continuous batching).
 //
 // Each ray is traced by exactly the code of the single-trace kernel
-// (trace_tile in tracer.cuh), so a job's results do not depend on which
+// (trace_warp in tracer.cuh), so a job's results do not depend on which
 // other jobs share its iterations.
 #include <atomic>
 #include <cstring>
@@ -50,59 +50,57 @@ struct WorkItem {
 };
 
 struct WorkHeader {
-    int counter[kModes];   // tiles taken so far (zero when the iteration starts)
+    int counter[kModes];   // shares of tiles taken so far (zero when the iteration starts)
     int count[kModes];     // tiles of each mode
     int offset[kModes];    // first item of each mode
     int pad;
 };
 
+// One warp per CTA. A warp takes kWarpRays consecutive rays of a work item's
+// tile at a time, so a tile's rays spread over as many warps as are free.
+constexpr int kTile = 1024;               // rays per work item
+constexpr int kWarpRays = 32;
+constexpr int kTileShares = kTile / kWarpRays;
+static_assert(kThreads == 32, "a serving CTA is one warp");
+
 template <int IB, int FAST>
 __global__ void __launch_bounds__(kThreads, SLOTH_TRACE_MIN_BLOCKS)
 serve_kernel(const TraceArgs* __restrict__ table, WorkHeader* hdr, const WorkItem* __restrict__ items, int mode) {
     __shared__ TraceArgs s_args;
-    __shared__ unsigned s_key[kTile];
-    __shared__ unsigned s_id[kTile];
-    __shared__ int s_item, s_slot, s_newslot, s_tile, s_head;
-    __shared__ unsigned long long s_steps;
     CellCacheFor<PolF32, IB> cc;
     cc.base = 0xffffffffu;
-    if (threadIdx.x == 0) {
-        s_slot = -1;
-        s_steps = 0;
-    }
-    const int count = hdr->count[mode];
+    int slot = -1;
+    const int shares = hdr->count[mode] * kTileShares;
     const int offset = hdr->offset[mode];
+    unsigned long long my_steps = 0;
     for (;;) {
-        if (threadIdx.x == 0) {
-            const int w = atomicAdd(&hdr->counter[mode], 1);
-            s_item = w;
-            s_head = 0;
-            if (w < count) {
-                const WorkItem it = items[offset + w];
-                s_tile = it.tile;
-                s_newslot = it.slot;
-            }
-        }
-        __syncthreads();
-        if (s_item >= count) break;
-        if (s_newslot != s_slot) {
+        int w = 0;
+        if (threadIdx.x == 0) w = atomicAdd(&hdr->counter[mode], 1);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (w >= shares) break;
+        const WorkItem it = items[offset + w / kTileShares];
+        if (it.slot != slot) {
             // a tile of another job: its arguments into shared memory, and
             // the cell cache no longer refers to the same grid
-            const unsigned* src = reinterpret_cast<const unsigned*>(table + s_newslot);
+            if (slot >= 0) warp_add(my_steps, s_args.total_steps);
+            my_steps = 0;
+            slot = it.slot;
+            __syncwarp();
+            const unsigned* src = reinterpret_cast<const unsigned*>(table + slot);
             unsigned* dst = reinterpret_cast<unsigned*>(&s_args);
-            for (int i = threadIdx.x; i < (int)(sizeof(TraceArgs) / 4); i += blockDim.x) dst[i] = src[i];
+            for (int i = threadIdx.x; i < (int)(sizeof(TraceArgs) / 4); i += 32) dst[i] = src[i];
             cc.base = 0xffffffffu;
-            __syncthreads();
-            if (threadIdx.x == 0) s_slot = s_newslot;
+            __syncwarp();
         }
-        const long long start = (long long)s_tile * kTile;
-        const int cnt = (int)min((long long)kTile, s_args.n - start);
-        unsigned long long my_steps = 0;
+        const unsigned start = (unsigned)it.tile * kTile + (unsigned)(w % kTileShares) * kWarpRays;
+        const unsigned n = (unsigned)s_args.n;
+        if (start >= n) continue;
+        RangeQueue q{start, min(start + kWarpRays, n)};
         // FAST: the job's density range bounds its accelerations (the host
         // sorted its tiles by interior_sampling_ok)
-        trace_tile<PolF32, IB, FAST>(s_args, start, cnt, s_key, s_id, &s_head, cc, my_steps);
-        block_add(my_steps, &s_steps, s_args.total_steps);
+        trace_warp<PolF32, IB, FAST>(s_args, q, cc, my_steps);
     }
+    if (slot >= 0) warp_add(my_steps, s_args.total_steps);
 }
 
 // ---------------------------------------------------------------------------
@@ -258,8 +256,8 @@ static size_t job_bytes(long long n, const SlothTraceParams* p, int* bbits_out, 
     sz[4] = align256(N);                          // status
     sz[5] = align256(N * 4);                      // steps
     sz[6] = 256;                                  // total steps
-    sz[7] = align256(((size_t)4 << bbits));       // histogram
-    sz[8] = align256(N * 4) * 3;                  // keys, perm, sorted keys
+    sz[7] = align256(hist_bytes(bbits));          // histogram
+    sz[8] = align256(N * 4) * 3;                  // keys, perm, bucket offsets
     size_t total = 0;
     for (int i = 0; i < 9; ++i) {
         if (parts) parts[i] = total;
@@ -400,14 +398,13 @@ static int admit_one(ServerImpl* s, Job& j) {
     const size_t an = align256((size_t)j.n * 4);
     unsigned* keys = reinterpret_cast<unsigned*>(base + parts[8]);
     unsigned* perm = reinterpret_cast<unsigned*>(base + parts[8] + an);
-    unsigned* skeys = reinterpret_cast<unsigned*>(base + parts[8] + 2 * an);
+    unsigned* offs = reinterpret_cast<unsigned*>(base + parts[8] + 2 * an);
     cudaError_t e = cudaMemcpyAsync(rays, j.rays_src, (size_t)j.n * 6 * 4,
                                     j.rays_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s->admit);
-    if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, (size_t)4 << bbits, s->admit);
-    if (e == cudaSuccess) e = cudaMemsetAsync(j.out.total_steps, 0, 8, s->admit);
+    if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, hist_bytes(bbits), s->admit);
     int rc = cuda_status(e);
-    if (!rc) rc = launch_prepass<float>(&ge->desc, j.p.probing_axis, rays, j.n, bbits, keys, hist, perm, skeys,
-                                        s->sms, s->admit);
+    if (!rc) rc = launch_prepass<float>(&ge->desc, j.p.probing_axis, rays, j.n, bbits, keys, hist, perm, offs,
+                                        j.out.total_steps, s->sms, s->admit);
     if (rc) {
         s->arena.release(off, bytes);
         --ge->refs;
@@ -416,7 +413,7 @@ static int admit_one(ServerImpl* s, Job& j) {
     j.slot = s->free_slots.back();
     s->free_slots.pop_back();
     TraceArgs& ta = s->h_table[j.slot];
-    fill_trace_args(ta, &ge->desc, s->arena.ptr(ge->off), &j.p, rays, j.n, &j.out, perm, skeys);
+    fill_trace_args(ta, &ge->desc, s->arena.ptr(ge->off), &j.p, rays, j.n, &j.out, perm);
     e = cudaMemcpyAsync(s->d_table + j.slot, &ta, sizeof(TraceArgs), cudaMemcpyHostToDevice, s->admit);
     if (e != cudaSuccess) return cuda_status(e);
     j.mode = 2 * trace_mode(&j.p) + (interior_sampling_ok(ta) ? 1 : 0);

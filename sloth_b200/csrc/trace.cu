@@ -1,47 +1,21 @@
 // K2 (FP32 split) and K3 (FP64 port) tracer entry points: one trace of one
 // ray set through one grid (the device code is in tracer.cuh).
-#include <algorithm>
-
 #include "tracer.cuh"
 
 namespace sloth {
 
 template <class P, int IB, int FAST, int INTEG>
 __global__ void __launch_bounds__(kThreads, SLOTH_TRACE_MIN_BLOCKS)
-trace_kernel(const __grid_constant__ TraceArgs a) {
-    __shared__ unsigned s_key[kTile];
-    __shared__ unsigned s_id[kTile];
-    __shared__ int s_tile, s_head;
-    __shared__ unsigned long long s_steps;
+trace_kernel(const __grid_constant__ TraceArgs a, int first_rays) {
     unsigned long long my_steps = 0;
-    if (threadIdx.x == 0) s_steps = 0;
     CellCacheFor<P, IB> cc;
     cc.base = 0xffffffffu;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            s_tile = atomicAdd(a.tile_counter, 1);
-            s_head = 0;
-        }
-        __syncthreads();
-        const int tile = s_tile;
-        if (tile >= a.n_tiles) break;
-        // Rays that start together in a tile have similar lifetimes, so a
-        // kTile tile runs as kTile / kThreads waves. The queue ends in tiles
-        // of one wave, so the CTAs finish within about one ray lifetime of
-        // each other instead of one tile.
-        long long start;
-        int cnt;
-        if (tile < a.n_big) {
-            start = (long long)tile * kTile;
-            cnt = kTile;
-        } else {
-            start = (long long)a.n_big * kTile + (long long)(tile - a.n_big) * kSmallTile;
-            cnt = (int)min((long long)kSmallTile, a.n - start);
-        }
-        trace_tile<P, IB, FAST, INTEG>(a, start, cnt, s_key, s_id, &s_head, cc, my_steps);
-    }
-    // one atomic per CTA for the ray-step total
-    block_add(my_steps, &s_steps, a.total_steps);
+    const unsigned n = (unsigned)a.n;
+    const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const unsigned warps = gridDim.x * (kThreads / 32);
+    TraceQueue q{a.queue, warps * first_rays, min(warp * first_rays, n), min((warp + 1) * first_rays, n), n};
+    trace_warp<P, IB, FAST, INTEG>(a, q, cc, my_steps);
+    warp_add(my_steps, a.total_steps);
 }
 
 template <class P, int IB, int FAST, int INTEG>
@@ -58,14 +32,10 @@ static int launch_trace_k(const TraceArgs& ta, int sms, cudaStream_t s) {
         if (dev >= 0 && dev < 64) cached[dev] = per_sm;
     }
     long long blocks = (long long)sms * per_sm;
-    // tile queue: big tiles, then the last kTailWaves small tiles per CTA
-    TraceArgs t = ta;
-    const long long small = std::min(ta.n, (long long)kTailWaves * blocks * kSmallTile);
-    t.n_big = (int)((ta.n - small) / kTile);
-    const long long rest = ta.n - (long long)t.n_big * kTile;
-    t.n_tiles = t.n_big + (int)((rest + kSmallTile - 1) / kSmallTile);
-    if (blocks > t.n_tiles) blocks = t.n_tiles;
-    trace_kernel<P, IB, FAST, INTEG><<<(int)blocks, kThreads, 0, s>>>(t);
+    const int first = 32;
+    const long long want = (ta.n + first * (kThreads / 32) - 1) / (first * (kThreads / 32));
+    if (blocks > want) blocks = want;
+    trace_kernel<P, IB, FAST, INTEG><<<(int)blocks, kThreads, 0, s>>>(ta, first);
     note_launch();
     return cuda_status(cudaGetLastError());
 }
@@ -106,30 +76,26 @@ static int trace_impl(const SlothGridDesc* g, const void* grid, const SlothTrace
 
     cudaStream_t s = (cudaStream_t)stream;
     char* base = reinterpret_cast<char*>(ws);
-    int* tile_counter = reinterpret_cast<int*>(base);
+    unsigned* queue = reinterpret_cast<unsigned*>(base);
     unsigned* hist = reinterpret_cast<unsigned*>(base + kHeaderBytes);
     const size_t an = align256((size_t)n * 4u);
     unsigned* keys = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes);
     unsigned* perm = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes + an);
-    unsigned* skeys = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes + 2 * an);
+    unsigned* offs = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes + 2 * an);
 
     const int bbits = bucket_bits_for(n);
-    cudaError_t e = cudaMemsetAsync(base, 0, kHeaderBytes + ((size_t)4 << bbits), s);
+    cudaError_t e = cudaMemsetAsync(base, 0, kHeaderBytes + hist_bytes(bbits), s);
     if (e != cudaSuccess) return cuda_status(e);
-    if (out->total_steps) {
-        e = cudaMemsetAsync(out->total_steps, 0, sizeof(unsigned long long), s);
-        if (e != cudaSuccess) return cuda_status(e);
-    }
     int sms = 148;
     rc = device_sm_count(&sms);
     if (rc) return rc;
     rc = launch_prepass<R>(g, p->probing_axis, reinterpret_cast<const R*>(rays), n, bbits, keys, hist, perm,
-                           skeys, sms, s);
+                           offs, out->total_steps, sms, s);
     if (rc) return rc;
 
     TraceArgs ta;
-    fill_trace_args(ta, g, grid, p, rays, n, out, perm, skeys);
-    ta.tile_counter = tile_counter;
+    fill_trace_args(ta, g, grid, p, rays, n, out, perm);
+    ta.queue = queue;
     const int ib = trace_mode(p);
     // interior runs with interior sampling, interior runs only, or neither
     const int fast = interior_bound_ok(g, p) ? 1 : (std::isfinite(interior_accel_bound(g, p)) ? 2 : 0);
@@ -154,7 +120,7 @@ static int trace_impl(const SlothGridDesc* g, const void* grid, const SlothTrace
 }
 
 // ---------------------------------------------------------------------------
-// Allocation-free variant of the FP32 tracer: its scratch (tile counter,
+// Allocation-free variant of the FP32 tracer: its scratch (ray counter,
 // bucket histogram, keys, permutation) lives in one file-scope device array
 // sized for SLOTH_NOALLOC_MAX_RAYS rays, so the caller passes only inputs and
 // outputs and nothing here allocates. Host code cannot use the array's name

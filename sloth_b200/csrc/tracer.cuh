@@ -26,25 +26,28 @@
 //
 // Launch structure (all on the caller's stream):
 //   1. keys_kernel   : Morton key of each ray's entry cell + bucket histogram
-//   2. scan_kernel   : exclusive scan of the bucket counts (one CTA)
-//   3. scatter_kernel: rays into bucket order
-//   4. trace_kernel  : persistent CTAs; each takes a tile of 1024 rays in
-//                      bucket order, sorts it by full key in shared memory,
-//                      and its warps trace the tile; lanes whose ray has
-//                      finished are refilled from the tile with one warp
-//                      ballot + one shared-memory atomic per refill.
+//   2. scan_kernel   : exclusive scan of the bucket counts
+//   3. scatter_kernel: ray ids into bucket order
+//   4. trace_kernel  : persistent one-warp CTAs; each warp traces 32
+//                      neighbouring rays of the bucket order, one thread per
+//                      ray, and refills finished lanes from the queue with one
+//                      warp ballot + one atomic (see trace_warp).
 #pragma once
 
+#include <climits>
 #include <cmath>
 #include <type_traits>
 
 #include "common.cuh"
 
 #ifndef SLOTH_TRACE_THREADS
-#define SLOTH_TRACE_THREADS 256
+#define SLOTH_TRACE_THREADS 32
 #endif
 #ifndef SLOTH_TRACE_MIN_BLOCKS
-#define SLOTH_TRACE_MIN_BLOCKS 2
+#define SLOTH_TRACE_MIN_BLOCKS 16
+#endif
+#ifndef SLOTH_REFILL
+#define SLOTH_REFILL 28
 #endif
 #ifndef SLOTH_PAIRED_F32
 #define SLOTH_PAIRED_F32 1
@@ -55,7 +58,8 @@
 
 namespace sloth {
 
-constexpr int kThreads = SLOTH_TRACE_THREADS;
+constexpr int kThreads = SLOTH_TRACE_THREADS;   // one warp per CTA
+constexpr int kRefill = SLOTH_REFILL;            // idle lanes that a warp refills together
 constexpr double kFaceMargin = 0.02;     // cells
 
 // Inverse-bremsstrahlung modes of the tracer.
@@ -90,10 +94,7 @@ struct TraceArgs {
     const void* rays;          // (6, N) of R
     long long n;
     const unsigned* perm;      // bucket-ordered ray ids
-    const unsigned* skeys;     // their keys
-    int* tile_counter;
-    int n_tiles;      // n_big tiles of kTile rays, then tiles of kSmallTile rays
-    int n_big;
+    unsigned* queue;           // rays handed out beyond each warp's first ones
     double origin[3], spacing[3];
     double w_of_v[3];          // w = v * w_of_v   (cells per step per m/s)
     double v_of_w[3];          // v = w * v_of_w
@@ -1137,76 +1138,77 @@ __device__ __forceinline__ bool start_ray(const TraceArgs& a, unsigned id, Ray<P
     return settle<P>(a, r, my_steps);
 }
 
-// Shared-memory bitonic sort of `size` (a power of two, <= kTile) (key, id)
-// pairs, ascending by key then id. `size` must be the same in every thread.
-__device__ __forceinline__ void tile_sort(unsigned* key, unsigned* id, int size) {
-    for (int k = 2; k <= size; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < size; i += blockDim.x) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const unsigned ki = key[i], kl = key[l], ii = id[i], il = id[l];
-                    const bool gt = (ki > kl) || (ki == kl && ii > il);
-                    const bool up = (i & k) == 0;
-                    if (gt == up) {
-                        key[i] = kl; key[l] = ki;
-                        id[i] = il; id[l] = ii;
-                    }
-                }
-            }
-            __syncthreads();
+// Ray queue of a whole trace: each warp first takes rays of its own
+// (`first` to `first_end`), then rays from the shared counter, which starts
+// behind the first rays of all the warps.
+struct TraceQueue {
+    unsigned* counter;
+    unsigned base0, first, first_end, n;
+    __device__ __forceinline__ bool take(int k, int lane, unsigned& base, unsigned& end) {
+        if (first < first_end) {
+            base = first;
+            end = first_end;
+            first = first_end;
+            return true;
         }
+        unsigned b = 0;
+        if (lane == 0) b = atomicAdd(counter, (unsigned)k);
+        base = base0 + __shfl_sync(0xffffffffu, b, 0);
+        end = min(base + (unsigned)k, n);
+        return base + (unsigned)k < n;
     }
-}
+};
 
-// Traces one tile of `cnt` rays (bucket-ordered ids perm[start..], keys
-// skeys[start..]): sorts them by key in shared memory, then the block's warps
-// trace them one thread per ray, refilling finished lanes from the tile
-// (warp ballot + shared-memory atomic). *s_head must be 0 on entry and the
-// block must be synchronised. Shared by the single-trace and serving kernels.
+// A run of rays known in advance (a serving tile's share).
+struct RangeQueue {
+    unsigned head, n;
+    __device__ __forceinline__ bool take(int k, int, unsigned& base, unsigned& end) {
+        base = head;
+        head += (unsigned)k;
+        end = min(head, n);
+        return head < n;
+    }
+};
+
+// Traces the rays of a queue, one thread per ray of this warp. `q.take(k)`
+// hands out up to k rays [base, end) of the bucket order and returns whether
+// more may follow. Shared by the single-trace and serving kernels.
+// Rays taken together start in neighbouring cells at the same place along the
+// beam, so the warp's cell fills stay together and its lanes finish within a
+// few steps of each other; a lane refilled in the middle would fill its cells
+// alone (a fill costs about a fifth of two steps) for the rest of its life.
+// So finished lanes wait until kRefill lanes are idle, which keeps one late
+// ray from holding the whole warp. 512^3 / 1e7 rays with 3 mm beams and 256^3 /
+// 1e6 rays with 6 mm beams (many side exits): 132.6 and - ms refilled one by one,
+// 117.1 and 5.21 at 8 idle lanes, 107.1 and 5.13 at 16, 105.4 and 5.13 at 24,
+// 104.7 and 5.20 at 30, 105.0 and 5.43 at 32. Nothing else synchronises: a CTA
+// is one warp, and no warp waits for another one's rays. (Tiles of 1024 rays,
+// sorted and traced by CTAs of eight warps that met at each tile's end, took
+// 110.7 ms; and a small trace's tiles kept most SMs idle: 1e4 rays through
+// 128^3 took 180 us in the kernel on 40 CTAs, 113 us on 313.)
 // FAST: 0 every step runs the face test; 1 steps proven interior by the
 // acceleration bound skip it and sample without the grid test (bound at most
 // kInteriorAccel); 2 they skip the face test but sample with the grid test
 // (any finite bound). Every mode takes the same steps.
-template <class P, int IB, int FAST, int INTEG = INTEG_RKN, class Cache>
-__device__ __forceinline__ void trace_tile(const TraceArgs& a, long long start, int cnt, unsigned* s_key,
-                                           unsigned* s_id, int* s_head, Cache& cc,
-                                           unsigned long long& my_steps) {
+template <class P, int IB, int FAST, int INTEG = INTEG_RKN, class Queue, class Cache>
+__device__ __forceinline__ void trace_warp(const TraceArgs& a, Queue& q, Cache& cc, unsigned long long& my_steps) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
-    int size = 32;                      // sort the smallest power of two that holds the tile
-    while (size < cnt) size <<= 1;
-    for (int i = threadIdx.x; i < size; i += blockDim.x) {
-        if (i < cnt) {
-            s_key[i] = a.skeys[start + i];
-            s_id[i] = a.perm[start + i];
-        } else {
-            s_key[i] = 0xffffffffu;
-            s_id[i] = 0xffffffffu;
-        }
-    }
-    __syncthreads();
-    tile_sort(s_key, s_id, size);
-
     Ray<P> r;
-    bool active = false, qempty = false;
+    bool active = false, more = true;
     for (;;) {
         const unsigned idle = __ballot_sync(FULL, !active);
-        if (idle != 0u && !qempty) {
-            const int nidle = __popc(idle);
-            const int leader = __ffs(idle) - 1;
-            int base = 0;
-            if (lane == leader) base = atomicAdd(s_head, nidle);
-            base = __shfl_sync(FULL, base, leader);
-            if (base + nidle >= cnt) qempty = true;
+        if (more && __popc(idle) >= kRefill) {
+            unsigned base, end;
+            more = q.take(__popc(idle), lane, base, end);
             if (!active) {
-                const int kk = base + __popc(idle & lt_mask);
-                if (kk < cnt) active = start_ray<P>(a, s_id[kk], r, my_steps);
+                const unsigned k = base + __popc(idle & lt_mask);
+                if (k < end) active = start_ray<P>(a, a.perm[k], r, my_steps);
             }
         }
         if (__ballot_sync(FULL, active) == 0u) {
-            if (qempty) break;
+            if (!more) break;
             continue;
         }
         typename P::R phi = typename P::R(1);
@@ -1220,13 +1222,14 @@ __device__ __forceinline__ void trace_tile(const TraceArgs& a, long long start, 
                 if (FAST && kind == 0) r.run = interior_run<P>(a, r);
             }
         }
-        // Fast path: when every lane takes an interior step, the warp takes
-        // `extra` more of them in a uniform loop, as many as every lane's run
-        // allows before its next save (so no save falls inside the loop and
-        // no lane needs the face test, the refill or settle in between).
+        // Fast path: when every live lane takes an interior step, the warp
+        // takes `extra` more of them in a uniform loop, as many as every such
+        // lane's run allows before its next save (so no save falls inside the
+        // loop and no lane needs the face test, the refill or settle in
+        // between). Idle lanes wait outside the minimum.
         int extra = 0;
         if (FAST) {
-            const int mine = kind == 0 ? min(r.run, r.next_save - r.step - 1) : 0;
+            const int mine = !active ? INT_MAX : (kind == 0 ? min(r.run, r.next_save - r.step - 1) : 0);
             extra = __reduce_min_sync(FULL, mine);
         }
         if (active) {
@@ -1252,7 +1255,6 @@ __device__ __forceinline__ void trace_tile(const TraceArgs& a, long long start, 
             active = settle<P>(a, r, my_steps, kind != 0);
         }
     }
-    __syncthreads();
 }
 
 // Register cache of the last cell: polynomial coefficients or corners.
@@ -1262,6 +1264,13 @@ using CellCacheFor = typename std::conditional<
     typename std::conditional<std::is_same<typename P::R, float>::value && SLOTH_PAIRED_F32,
                               CellPolyF2<(IB != IB_OFF) ? 5 : 4>, CellPoly<P, (IB != IB_OFF) ? 5 : 4>>::type,
     CellCache<P>>::type;
+
+// Sum of `v` over the warp, added to *dst by one lane.
+__device__ __forceinline__ void warp_add(unsigned long long v, unsigned long long* dst) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0 && v && dst) atomicAdd(dst, v);
+}
 
 // Sum of `v` over the block, added to *dst by one thread.
 __device__ __forceinline__ void block_add(unsigned long long v, unsigned long long* s_acc,
@@ -1314,94 +1323,79 @@ __global__ void __launch_bounds__(256) keys_kernel(const KeyArgs k) {
     }
 }
 
-// Exclusive scan of nb (<= 2^18) counts by one CTA of 1024 threads, in
-// passes of 16384 counts: each thread takes 16 consecutive counts (four
-// 16-byte loads; hist is 256-byte aligned), the block scans the per-thread
-// sums, and a running carry links the passes. The next pass's counts are
-// loaded before this pass's block scan, so their latency overlaps it.
+// Exclusive scan of nb (<= 2^18) counts into offs, kScanSeg counts per CTA.
+// Each CTA first sums every count before its segment, so that no CTA waits
+// for another and one launch does it: at 2^18 counts the last of 64 CTAs
+// reads 1 MB through L2 (one CTA alone: 56 us). hist and offs are 16-byte aligned and padded to a
+// multiple of four counts; hist's padding is zero.
+constexpr int kScanThreads = 256;
 constexpr int kScanPer = 16;
-constexpr int kScanPass = 1024 * kScanPer;
+constexpr int kScanSeg = kScanThreads * kScanPer;
 
-__device__ __forceinline__ void scan_load(const unsigned* hist, int nb, int i0, unsigned (&x)[kScanPer]) {
-    if (i0 + kScanPer <= nb) {
-        const uint4* h4 = reinterpret_cast<const uint4*>(hist + i0);
+__device__ __forceinline__ unsigned scan_block_sum(unsigned v, unsigned* s_warp) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    v = __reduce_add_sync(0xffffffffu, v);
+    __syncthreads();
+    if (lane == 0) s_warp[wid] = v;
+    __syncthreads();
+    unsigned t = 0;
 #pragma unroll
-        for (int q = 0; q < kScanPer / 4; ++q) {
-            const uint4 u = h4[q];
-            x[4 * q] = u.x;
-            x[4 * q + 1] = u.y;
-            x[4 * q + 2] = u.z;
-            x[4 * q + 3] = u.w;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < kScanPer; ++j) x[j] = i0 + j < nb ? hist[i0 + j] : 0u;
-    }
+    for (int k = 0; k < kScanThreads / 32; ++k) t += s_warp[k];
+    return t;
 }
 
-static __global__ void __launch_bounds__(1024) scan_kernel(unsigned* hist, int nb) {
-    __shared__ unsigned s_warp[32];
+static __global__ void __launch_bounds__(kScanThreads) scan_kernel(const unsigned* __restrict__ hist,
+                                                                   unsigned* __restrict__ offs, int nb,
+                                                                   unsigned long long* zero) {
+    __shared__ unsigned s_warp[kScanThreads / 32];
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    unsigned v[kScanPer], nx[kScanPer];
-    scan_load(hist, nb, t * kScanPer, v);
-    unsigned carry = 0;
-    for (int base = 0; base < nb; base += kScanPass) {
-        const int i0 = base + t * kScanPer;
-        if (base + kScanPass < nb) scan_load(hist, nb, i0 + kScanPass, nx);
-        unsigned sum = 0;
-#pragma unroll
-        for (int j = 0; j < kScanPer; ++j) {
-            const unsigned c = v[j];
-            v[j] = sum;
-            sum += c;
-        }
-        unsigned inc = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += y;
-        }
-        if (lane == 31) s_warp[wid] = inc;
-        __syncthreads();
-        if (wid == 0) {
-            unsigned w = s_warp[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
-            }
-            s_warp[lane] = w;
-        }
-        __syncthreads();
-        const unsigned excl = carry + (inc - sum) + (wid > 0 ? s_warp[wid - 1] : 0u);
-        carry += s_warp[31];
-        if (i0 + kScanPer <= nb) {
-            uint4* h4 = reinterpret_cast<uint4*>(hist + i0);
-#pragma unroll
-            for (int q = 0; q < kScanPer / 4; ++q)
-                h4[q] = make_uint4(v[4 * q] + excl, v[4 * q + 1] + excl, v[4 * q + 2] + excl, v[4 * q + 3] + excl);
-        } else {
-#pragma unroll
-            for (int j = 0; j < kScanPer; ++j)
-                if (i0 + j < nb) hist[i0 + j] = v[j] + excl;
-        }
-        __syncthreads();   // s_warp is rewritten by the next pass
-#pragma unroll
-        for (int j = 0; j < kScanPer; ++j) v[j] = nx[j];
+    const int seg = blockIdx.x * kScanSeg;
+    if (zero && blockIdx.x == 0 && t == 0) *zero = 0ull;
+    const uint4* h4 = reinterpret_cast<const uint4*>(hist);
+    unsigned before = 0;
+#pragma unroll 8
+    for (int i = t; i < seg / 4; i += kScanThreads) {
+        const uint4 u = __ldg(h4 + i);
+        before += (u.x + u.y) + (u.z + u.w);
     }
+    const unsigned carry = scan_block_sum(before, s_warp);
+    const int i0 = seg + t * kScanPer;
+    unsigned v[kScanPer];
+    unsigned sum = 0;
+#pragma unroll
+    for (int q = 0; q < kScanPer / 4; ++q) {
+        uint4 u = make_uint4(0u, 0u, 0u, 0u);
+        if (i0 + 4 * q < nb) u = __ldg(h4 + i0 / 4 + q);
+        v[4 * q] = sum;
+        v[4 * q + 1] = v[4 * q] + u.x;
+        v[4 * q + 2] = v[4 * q + 1] + u.y;
+        v[4 * q + 3] = v[4 * q + 2] + u.z;
+        sum = v[4 * q + 3] + u.w;
+    }
+    unsigned inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    __syncthreads();
+    if (lane == 31) s_warp[wid] = inc;
+    __syncthreads();
+    unsigned excl = carry + (inc - sum);
+    for (int k = 0; k < wid; ++k) excl += s_warp[k];
+#pragma unroll
+    for (int q = 0; q < kScanPer / 4; ++q)
+        if (i0 + 4 * q < nb)
+            reinterpret_cast<uint4*>(offs)[i0 / 4 + q] =
+                make_uint4(v[4 * q] + excl, v[4 * q + 1] + excl, v[4 * q + 2] + excl, v[4 * q + 3] + excl);
 }
 
 static __global__ void __launch_bounds__(256) scatter_kernel(const unsigned* __restrict__ keys, long long n,
                                                       int bucket_shift, unsigned* offs,
-                                                      unsigned* __restrict__ perm,
-                                                      unsigned* __restrict__ skeys) {
+                                                      unsigned* __restrict__ perm) {
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const unsigned key = keys[i];
-        const unsigned pos = atomicAdd(offs + (key >> bucket_shift), 1u);
-        perm[pos] = (unsigned)i;
-        skeys[pos] = key;
-    }
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+        perm[atomicAdd(offs + (keys[i] >> bucket_shift), 1u)] = (unsigned)i;
 }
 
 // ---------------------------------------------------------------------------
@@ -1417,23 +1411,33 @@ inline size_t workspace_bytes(long long n) {
     return kHeaderBytes + kHistBytes + 3 * a;
 }
 
+// Buckets of the pre-pass: about one per kBucketRays rays, at most 2^18. The
+// histogram takes kHistBytes of the workspace and its scan the n words
+// behind the permutation (2^bits < n / 4 for n > kBucketRays).
+constexpr int kBucketRays = 8;
 inline int bucket_bits_for(long long n) {
     int bits = 0;
-    while (bits < kMaxBucketBits && ((long long)1 << bits) * 32 < n) ++bits;
+    while (bits < kMaxBucketBits && ((long long)1 << bits) * kBucketRays < n) ++bits;
     return bits;
 }
 
+// Bytes of the histogram that the caller zeroes (the scan reads whole uint4).
+inline size_t hist_bytes(int bbits) { return bbits < 2 ? 16 : (size_t)4 << bbits; }
 
 // Morton pre-pass of n rays into bucket order: keys, histogram (2^bbits
-// buckets, zeroed by the caller), exclusive scan, scatter into perm/skeys.
-// The buckets are the keys' top bbits bits; with fine_buckets, the top bbits
-// of the bits the grid's keys use, so that a small grid's transverse cells
-// get buckets of their own (for kernels that trace rays in bucket order
-// without a further sort).
+// buckets, zeroed by the caller), exclusive scan, scatter into perm. `offs`
+// holds max(4, 2^bbits) words; *zero (may be null) is set to 0 on the way.
+// The buckets are the top bbits bits of those bits that the grid's keys use:
+// with few rays per bucket a warp's 32 rays come from one or two neighbouring
+// buckets, which needs no further sort, and the atomics spread over as many
+// words. (The top bits of the whole 30-bit key, most of which a grid of 2^8
+// cells leaves at zero, put 217k rays into 512 buckets: 40 us each for the
+// histogram and the scatter against 4 us, and a sort per tile of 1024 rays in
+// the tracer.)
 template <class R>
 inline int launch_prepass(const SlothGridDesc* g, int axis, const R* rays, long long n, int bbits,
-                          unsigned* keys, unsigned* hist, unsigned* perm, unsigned* skeys, int sms,
-                          cudaStream_t s, bool fine_buckets = false) {
+                          unsigned* keys, unsigned* hist, unsigned* perm, unsigned* offs,
+                          unsigned long long* zero, int sms, cudaStream_t s) {
     const int t1 = axis == 0 ? 1 : 0;
     const int t2 = axis == 2 ? 1 : 2;
     KeyArgs ka;
@@ -1450,23 +1454,21 @@ inline int launch_prepass(const SlothGridDesc* g, int axis, const R* rays, long 
     ka.axis = axis;
     ka.t1 = t1;
     ka.t2 = t2;
-    ka.bucket_shift = 30 - bbits;
-    if (fine_buckets) {
-        int tb = 0;   // bits of the largest transverse cell coordinate
-        for (int t : {t1, t2})
-            while (((g->n[t] - 2) >> ka.shift[t]) >> tb) ++tb;
-        const int used = 2 * tb + 10;
-        ka.bucket_shift = used > bbits ? used - bbits : 0;
-    }
+    int tb = 0;   // bits of the largest transverse cell coordinate
+    for (int t : {t1, t2})
+        while (((g->n[t] - 2) >> ka.shift[t]) >> tb) ++tb;
+    const int used = 2 * tb + 10;
+    ka.bucket_shift = used > bbits ? used - bbits : 0;
     ka.keys = keys;
     ka.hist = hist;
     const long long nblk = (n + 255) / 256;
     const int kb = (int)(nblk < (long long)sms * 8 ? nblk : (long long)sms * 8);
+    const int nb = 1 << bbits;
     keys_kernel<R><<<kb, 256, 0, s>>>(ka);
     note_launch();
-    scan_kernel<<<1, 1024, 0, s>>>(hist, 1 << bbits);
+    scan_kernel<<<(nb + kScanSeg - 1) / kScanSeg, kScanThreads, 0, s>>>(hist, offs, nb, zero);
     note_launch();
-    scatter_kernel<<<kb, 256, 0, s>>>(keys, n, ka.bucket_shift, hist, perm, skeys);
+    scatter_kernel<<<kb, 256, 0, s>>>(keys, n, ka.bucket_shift, offs, perm);
     note_launch();
     return cuda_status(cudaGetLastError());
 }
@@ -1492,18 +1494,14 @@ inline double interior_accel_bound(const SlothGridDesc* g, const SlothTraceParam
 
 // Kernel arguments of one trace from the public descriptors.
 inline void fill_trace_args(TraceArgs& ta, const SlothGridDesc* g, const void* grid, const SlothTraceParams* p,
-                            const void* rays, long long n, const SlothTraceOutputs* out, const unsigned* perm,
-                            const unsigned* skeys) {
+                            const void* rays, long long n, const SlothTraceOutputs* out, const unsigned* perm) {
     const int axis = p->probing_axis;
     ta.geo = make_geo(g);
     ta.grid = grid;
     ta.rays = rays;
     ta.n = n;
     ta.perm = perm;
-    ta.skeys = skeys;
-    ta.tile_counter = nullptr;
-    ta.n_tiles = (int)((n + kTile - 1) / kTile);
-    ta.n_big = ta.n_tiles;
+    ta.queue = nullptr;
     for (int k = 0; k < 3; ++k) {
         const double h = g->spacing[k];
         ta.origin[k] = g->origin[k];

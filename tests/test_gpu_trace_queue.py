@@ -1,0 +1,42 @@
+"""The tracer's ray queue and pre-pass at the sizes where they change: part
+of a warp, one ray around whole warps and around the rays that a full GPU's
+warps take first, and around the pre-pass's bucket counts (a scan of one word,
+of one and of several CTAs). Each ray's result does not depend on the other rays of its
+launch, so every size gives bitwise the rays of one larger trace."""
+import pytest
+import torch
+
+from sloth_b200 import runtime, workloads
+from sloth_b200.core import physics
+
+pytestmark = pytest.mark.gpu
+
+L = 5e-3
+
+
+def _trace(n_rays, rays, grid, sched, **kw):
+    o = {k: torch.full(s, v, dtype=d, device="cuda") for k, s, d, v in (
+        ("jones", (sched.n_saves, 4, n_rays), rays.dtype, 7e9), ("phase", (sched.n_saves, n_rays), torch.float64, 7e9),
+        ("status", (n_rays,), torch.uint8, 99), ("steps", (n_rays,), torch.int32, -5))}
+    return runtime.trace(grid, rays[:, :n_rays].contiguous(), sched, outputs=o, **kw)
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("shape", [(20, 33, 24), (2, 2, 40)])
+def test_every_ray_once_and_bitwise_the_same(precision, shape):
+    h = tuple(L / (k - 1) for k in shape)
+    g = torch.Generator().manual_seed(3)
+    ne = (torch.rand(shape, generator=g) * 2e25).float()
+    grid = runtime.pack_grid(ne, (-L / 2,) * 3, h, physics.omega_of(532e-9), precision=precision)
+    most = 148 * 16 * 32 + 33            # a B200's warps at 16 per SM, and one more warp's worth
+    rays = workloads.gaussian_beam(most, waist=3e-3, L=L, jitter=5e-2, seed=2, device="cuda", dtype=torch.float64)
+    rays = rays.to(torch.float32 if precision == "f32" else torch.float64)
+    sched = runtime.schedule_times([0.0, L, 2 * L], h)
+    whole = _trace(most, rays, grid, sched)
+    assert int(whole["total_steps"]) == int(whole["steps"].sum(dtype=torch.int64))
+    for n in (1, 2, 8, 9, 31, 32, 33, 64, 255, 257, 32768, 32769, 65537, 148 * 12 * 32 + 1, most - 33, most - 1):
+        part = _trace(n, rays, grid, sched)
+        for k in ("jones", "phase", "status", "steps"):
+            assert torch.equal(part[k], whole[k][..., :n]), (n, k)
+        assert int(part["total_steps"]) == int(part["steps"].sum(dtype=torch.int64))
+    assert int(whole["status"].max()) <= 2 and float(whole["jones"].abs().max()) < 1e9
