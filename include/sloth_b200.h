@@ -157,6 +157,14 @@ int sloth_grid_pack_trace_f32(const SlothGridDesc* g, const void* ne, int ne_is_
                               double ope_ratio2, void* grid_out, void* stream);
 int sloth_grid_pack_trace_f64(const SlothGridDesc* g, const void* ne, int ne_is_f64, double ne_scale,
                               double ope_ratio2, void* grid_out, void* stream);
+/* Either layout (trace for ope_ratio2 > 0, value for 0; element type by
+ * out_is_f64), with the density's range found on the way: range[0] receives
+ * the order key of the largest ne and range[1] that of the largest -ne (two
+ * device words, 8-byte aligned). The key of a double with bits b is b with the top bit set
+ * for b >= 0 and ~b otherwise, so that larger values have larger keys; if any
+ * ne is NaN both are all ones. */
+int sloth_grid_pack_range(const SlothGridDesc* g, const void* ne, int ne_is_f64, int out_is_f64, double ne_scale,
+                          double ope_ratio2, void* grid_out, unsigned long long* range, void* stream);
 
 /* ---- K0: trilinear sample -----------------------------------------------
  * Replaces RegularGridInterpolator (src/core/interpolator.py:15-105) on the

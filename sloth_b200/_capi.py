@@ -134,6 +134,8 @@ _SIGNATURES = {
                                           c_void_p]),
     "sloth_grid_pack_trace_f64": (c_int, [POINTER(SlothGridDesc), c_void_p, c_int, c_double, c_double, c_void_p,
                                           c_void_p]),
+    "sloth_grid_pack_range": (c_int, [POINTER(SlothGridDesc), c_void_p, c_int, c_int, c_double, c_double, c_void_p,
+                                      c_void_p, c_void_p]),
     "sloth_sample_f32": (c_int, [POINTER(SlothGridDesc), c_void_p, c_void_p, c_int64, c_void_p, c_void_p]),
     "sloth_sample_f64": (c_int, [POINTER(SlothGridDesc), c_void_p, c_void_p, c_int64, c_void_p, c_void_p]),
     "sloth_trace_workspace_bytes": (c_size_t, [c_int64]),

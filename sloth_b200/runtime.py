@@ -8,6 +8,7 @@ device the library returns an error and ``SlothError`` is raised.
 from __future__ import annotations
 
 import math
+import struct
 from dataclasses import dataclass
 from typing import Optional
 
@@ -81,6 +82,15 @@ class DeviceGrid:
         return tuple(o + h * (k - 1) for o, h, k in zip(self.origin, self.spacing, self.n))
 
 
+def _from_order_key(key: int) -> float:
+    """The double of an order key of sloth_grid_pack_range (as int64)."""
+    b = key & 0xFFFFFFFFFFFFFFFF
+    if b == 0xFFFFFFFFFFFFFFFF:
+        return float("nan")
+    b = b ^ (1 << 63) if b >> 63 else b ^ 0xFFFFFFFFFFFFFFFF
+    return struct.unpack("<d", struct.pack("<Q", b))[0]
+
+
 def pack_grid(ne, origin, spacing, omega, *, precision="f32", device=None, stream=None,
               out: Optional[torch.Tensor] = None, ne_scale: Optional[float] = None,
               layout: str = "trace") -> DeviceGrid:
@@ -114,20 +124,16 @@ def pack_grid(ne, origin, spacing, omega, *, precision="f32", device=None, strea
         out = torch.empty(nbytes // rb, dtype=torch.float32 if rb == 4 else torch.float64, device=dev)
     scale = 1.0 / physics.critical_density(omega) if ne_scale is None else float(ne_scale)
     lib = capi.load()
-    if layout == "trace":
-        fn = lib.sloth_grid_pack_trace_f32 if precision == "f32" else lib.sloth_grid_pack_trace_f64
-        capi.check(fn(desc, capi.ptr(ne), int(ne.dtype == torch.float64), scale, physics.ope_ratio2(omega),
-                      capi.ptr(out), _stream_ptr(stream)), "sloth_grid_pack_trace")
-    else:
-        fn = lib.sloth_grid_pack_f32 if precision == "f32" else lib.sloth_grid_pack_f64
-        capi.check(fn(desc, capi.ptr(ne), int(ne.dtype == torch.float64), scale, capi.ptr(out),
-                      _stream_ptr(stream)), "sloth_grid_pack")
-    if ne.numel():
-        lo, hi = torch.aminmax(ne)
-        ne_max = float(hi)
-        q_max, q_min = ne_max * scale, float(lo) * scale
-    else:
-        ne_max, q_max, q_min = 0.0, 0.0, 0.0
+    run_on = stream if stream is not None else torch.cuda.current_stream(dev)
+    if stream is not None:
+        run_on.wait_stream(torch.cuda.current_stream(dev))   # ne and out belong to the current stream
+    with torch.cuda.stream(run_on):
+        rng = torch.empty(2, dtype=torch.int64, device=dev)
+        capi.check(lib.sloth_grid_pack_range(desc, capi.ptr(ne), int(ne.dtype == torch.float64), int(rb == 8), scale,
+                                             physics.ope_ratio2(omega) if layout == "trace" else 0.0, capi.ptr(out),
+                                             capi.ptr(rng), _stream_ptr(run_on)), "sloth_grid_pack_range")
+        ne_max, neg_min = (_from_order_key(k) for k in rng.tolist())   # the one wait of the call
+    q_max, q_min = ne_max * scale, -neg_min * scale
     return DeviceGrid(out, desc, precision, float(omega), n, tuple(map(float, origin)), tuple(map(float, spacing)),
                       q_max=max(q_max, 0.0) * (1.0 + 1e-6), q_min=min(q_min, 0.0) * (1.0 + 1e-6), ne_max=ne_max,
                       layout=layout)
