@@ -87,28 +87,10 @@ struct AccD {
 struct Vox4F { float x, y, z, w; };
 struct Vox4D { double x, y, z, w; };
 
-#ifndef SLOTH_CELL_CACHE_F32
-#define SLOTH_CELL_CACHE_F32 1
-#endif
-#ifndef SLOTH_CELL_CACHE_F64
-#define SLOTH_CELL_CACHE_F64 1
-#endif
-#ifndef SLOTH_CELL_POLY_F32
-#define SLOTH_CELL_POLY_F32 1
-#endif
-#ifndef SLOTH_CELL_POLY_F64
-#define SLOTH_CELL_POLY_F64 0
-#endif
-
 struct PolF32 {
     using R = float;
     using V = Vox4F;
     using Acc = AccF;
-    // keep the last cell's 8 corners in registers across stages and steps
-    static constexpr bool cell_cache = SLOTH_CELL_CACHE_F32 != 0;
-    // keep the cached cell as trilinear polynomial coefficients (7 FMAs per
-    // channel per sample instead of 8 products and an 8-term sum)
-    static constexpr bool cell_poly = SLOTH_CELL_POLY_F32 != 0;
     __device__ __forceinline__ static V load(const void* g, unsigned i) {
         const float4 v = __ldg(reinterpret_cast<const float4*>(g) + i);
         return V{v.x, v.y, v.z, v.w};
@@ -120,8 +102,6 @@ struct PolF64 {
     using R = double;
     using V = Vox4D;
     using Acc = AccD;
-    static constexpr bool cell_cache = SLOTH_CELL_CACHE_F64 != 0;
-    static constexpr bool cell_poly = SLOTH_CELL_POLY_F64 != 0;
     __device__ __forceinline__ static V load(const void* g, unsigned i) {
         const double2* p = reinterpret_cast<const double2*>(g) + 2u * (size_t)i;
         const double2 a = __ldg(p), b = __ldg(p + 1);

@@ -67,7 +67,7 @@ template <int IB, int FAST>
 __global__ void __launch_bounds__(kThreads, SLOTH_TRACE_MIN_BLOCKS)
 serve_kernel(const TraceArgs* __restrict__ table, WorkHeader* hdr, const WorkItem* __restrict__ items, int mode) {
     __shared__ TraceArgs s_args;
-    CellCacheFor<PolF32, IB> cc;
+    CellCacheFor<PolF32> cc;
     cc.base = 0xffffffffu;
     int slot = -1;
     const int shares = hdr->count[mode] * kTileShares;

@@ -5,10 +5,10 @@
 namespace sloth {
 
 template <class P, int IB, int FAST, int INTEG>
-__global__ void __launch_bounds__(kThreads, SLOTH_TRACE_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, trace_min_blocks<P, INTEG>())
 trace_kernel(const __grid_constant__ TraceArgs a, int first_rays) {
     unsigned long long my_steps = 0;
-    CellCacheFor<P, IB> cc;
+    CellCacheFor<P> cc;
     cc.base = 0xffffffffu;
     const unsigned n = (unsigned)a.n;
     const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);

@@ -49,13 +49,6 @@
 #ifndef SLOTH_REFILL
 #define SLOTH_REFILL 28
 #endif
-#ifndef SLOTH_PAIRED_F32
-#define SLOTH_PAIRED_F32 1
-#endif
-#ifndef SLOTH_PAIRED_STEP
-#define SLOTH_PAIRED_STEP 1
-#endif
-
 namespace sloth {
 
 constexpr int kThreads = SLOTH_TRACE_THREADS;   // one warp per CTA
@@ -159,12 +152,6 @@ struct Ray {
     bool exited;               // left the grid through a face-clipped step
 };
 
-template <class P>
-struct CellCache {
-    unsigned base;
-    typename P::V c[8];
-};
-
 // One field sample: n - 1 (the trace layout's channel 0), the three gradient
 // channels and the inverse-bremsstrahlung rate per kappa_q2.
 template <class P>
@@ -172,14 +159,17 @@ struct Sample {
     typename P::R n1, g0, g1, g2, k;
 };
 
-// A cached cell as trilinear polynomials in the in-cell coordinates
-// (fx, fy, fz): per channel T = a + bx fx + by fy + bz fz + cxy fx fy +
-// cxz fx fz + cyz fy fz + cxyz fx fy fz, channels q, dq/du, dq/dv, dq/dw and
-// (when NK = 5) the inverse-bremsstrahlung corner rate.
-template <class P, int NK>
-struct CellPoly {
+// The cell cache: the last cell as trilinear polynomials in the in-cell
+// coordinates (fx, fy, fz), kept across stages and steps. Per channel T = a +
+// bx fx + by fy + bz fz + cxy fx fy + cxz fx fz + cyz fy fz + cxyz fx fy fz,
+// channels n - 1, dq/du, dq/dv, dq/dw in registers and the inverse-
+// bremsstrahlung corner rate in shared memory (see kappa_store): seven
+// multiply-adds per channel and sample. In FP64 the eight corners with the
+// weights rebuilt at each sample (about 79 FP64 operations with the rate against 35)
+// took 5.80 ms for 256^3 / 4e5 rays, the polynomials 4.53 ms.
+struct CellPolyD {
     unsigned base;
-    typename P::R t[NK][8];
+    double t[4][8];
 };
 
 template <class R>
@@ -213,26 +203,46 @@ __device__ __forceinline__ R poly_eval(const R (&t)[8], R fx, R fy, R fz) {
 // register pairs; each pair of trilinear polynomials is built and evaluated
 // with sm_100's two-wide FP32 instructions (__fadd2/__ffma2: one instruction
 // for two channels, each component rounded exactly as the scalar operation).
-// The inverse-bremsstrahlung channel (NK = 5) stays scalar.
-template <int NK>
+// The inverse-bremsstrahlung channel stays scalar.
 struct CellPolyF2 {
     unsigned base;
     float2 t[2][8];
 };
 
-// The FP32 paired cache keeps the cell's kappa polynomial (NK == 5) in shared
-// memory rather than registers: each thread owns one slot, [2][threads]
-// float4 so that a warp's 16-byte loads do not conflict. This keeps 8 values
-// out of the step's 128-register budget; the coefficients are written once
-// per cell and read once per stage, off the step's critical path.
+// The cell's kappa polynomial stays in shared memory rather than registers:
+// each thread owns one slot, [2][threads] float4 (FP64: [4][threads] double2) so
+// that a warp's 16-byte loads do not conflict. This keeps 8 values out of the
+// step's register budget; the coefficients are written once per cell and
+// read once per stage, off the step's critical path.
 static __shared__ float4 s_kappa_coef[2][kThreads];
+static __shared__ double2 s_kappa_coefd[4][kThreads];
 
 __device__ __forceinline__ void kappa_store(const float (&k)[8]) {
     s_kappa_coef[0][threadIdx.x] = make_float4(k[0], k[1], k[2], k[3]);
     s_kappa_coef[1][threadIdx.x] = make_float4(k[4], k[5], k[6], k[7]);
 }
 
-__device__ __forceinline__ float kappa_eval(float fx, float fy, float fz);
+__device__ __forceinline__ void kappa_store(const double (&k)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s_kappa_coefd[i][threadIdx.x] = make_double2(k[2 * i], k[2 * i + 1]);
+}
+
+__device__ __forceinline__ float kappa_eval(float fx, float fy, float fz) {
+    const float4 a = s_kappa_coef[0][threadIdx.x], b = s_kappa_coef[1][threadIdx.x];
+    const float k[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    return poly_eval<float>(k, fx, fy, fz);
+}
+
+__device__ __forceinline__ double kappa_eval(double fx, double fy, double fz) {
+    double k[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double2 v = s_kappa_coefd[i][threadIdx.x];
+        k[2 * i] = v.x;
+        k[2 * i + 1] = v.y;
+    }
+    return poly_eval<double>(k, fx, fy, fz);
+}
 
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
     return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);          // a - b, one rounding
@@ -257,9 +267,6 @@ __device__ __forceinline__ float2 poly_eval2(const float2 (&t)[8], float2 fx, fl
     const float2 cy = __ffma2_rn(fx, t[4], t[2]);
     return __ffma2_rn(fz, cz, __ffma2_rn(fy, cy, __ffma2_rn(fx, t[1], t[0])));
 }
-
-template <class C> struct IsPairedCache : std::false_type {};
-template <int NK> struct IsPairedCache<CellPolyF2<NK>> : std::true_type {};
 
 // x = (omega_pe/omega)^2 of a grid point from its n - 1 (the trace layout):
 // n - 1 = sqrt(1 - x) - 1 gives x = -(n - 1)(2 + (n - 1)) up to the critical
@@ -295,8 +302,8 @@ __device__ __forceinline__ R corner_x2(R n1) {
 
 // Loads cell b into the paired cache: its polynomial coefficients, two
 // channels per instruction.
-template <class P, int IB, int NK>
-__device__ __forceinline__ void paired_fill(const TraceArgs& a, unsigned b, CellPolyF2<NK>& cc) {
+template <class P, int IB>
+__device__ __forceinline__ void paired_fill(const TraceArgs& a, unsigned b, CellPolyF2& cc) {
     const GridGeo& g = a.geo;
     cc.base = b;
     const float4* gp = reinterpret_cast<const float4*>(a.grid);
@@ -326,13 +333,7 @@ __device__ __forceinline__ void paired_fill(const TraceArgs& a, unsigned b, Cell
     }
 }
 
-__device__ __forceinline__ float kappa_eval(float fx, float fy, float fz) {
-    const float4 a = s_kappa_coef[0][threadIdx.x], b = s_kappa_coef[1][threadIdx.x];
-    const float k[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    return poly_eval<float>(k, fx, fy, fz);
-}
-
-// Trilinear sample of the packed grid (rules of src/core/interpolator.py:79-104:
+// FP64 trilinear sample of the packed grid (rules of src/core/interpolator.py:79-104:
 // cell i = floor(p) clamped to [0, n-2], product weights, fill 0 outside)
 // returning q, the three gradient channels and, when IB, the interpolated
 // inverse-bremsstrahlung rate per kappa_q2. The reference interpolates a
@@ -386,108 +387,35 @@ __device__ __forceinline__ void sample_c(const TraceArgs& a, const typename P::R
     }
     const R fx = (h[0] - (R)ix) + l[0], fy = (h[1] - (R)iy) + l[1], fz = (h[2] - (R)iz) + l[2];
     const unsigned b = (unsigned)ix * g.sx + (unsigned)iy * g.sy + (unsigned)iz;
-    if constexpr (IsPairedCache<Cache>::value) {
-        if (b != cc.base) paired_fill<P, IB>(a, b, cc);
-        const float2 fx2 = make_float2(fx, fx), fy2 = make_float2(fy, fy), fz2 = make_float2(fz, fz);
-        const float2 r0 = poly_eval2(cc.t[0], fx2, fy2, fz2);
-        const float2 r1 = poly_eval2(cc.t[1], fx2, fy2, fz2);
-        out.n1 = r0.x;
-        out.g0 = r0.y;
-        out.g1 = r1.x;
-        out.g2 = r1.y;
+    if (b != cc.base) {
+        cc.base = b;
+        const V v0 = P::load(a.grid, b), v1 = P::load(a.grid, b + 1u);
+        const V v2 = P::load(a.grid, b + g.sy), v3 = P::load(a.grid, b + g.sy + 1u);
+        const V v4 = P::load(a.grid, b + g.sx), v5 = P::load(a.grid, b + g.sx + 1u);
+        const V v6 = P::load(a.grid, b + g.sx + g.sy), v7 = P::load(a.grid, b + g.sx + g.sy + 1u);
+        poly_coeffs<R>(cc.t[0], v0.x, v1.x, v2.x, v3.x, v4.x, v5.x, v6.x, v7.x);
+        poly_coeffs<R>(cc.t[1], v0.y, v1.y, v2.y, v3.y, v4.y, v5.y, v6.y, v7.y);
+        poly_coeffs<R>(cc.t[2], v0.z, v1.z, v2.z, v3.z, v4.z, v5.z, v6.z, v7.z);
+        poly_coeffs<R>(cc.t[3], v0.w, v1.w, v2.w, v3.w, v4.w, v5.w, v6.w, v7.w);
         if constexpr (IB == IB_SUBCRITICAL) {
-            out.k = kappa_eval(fx, fy, fz);   // cl_lo / ope2^2 is in tau_scale
+            R k[8];
+            poly_coeffs<R>(k, corner_x2(v0.x), corner_x2(v1.x), corner_x2(v2.x), corner_x2(v3.x), corner_x2(v4.x),
+                           corner_x2(v5.x), corner_x2(v6.x), corner_x2(v7.x));
+            kappa_store(k);
         } else if constexpr (IB == IB_GENERAL) {
-            out.k = kappa_eval(fx, fy, fz);
-        } else {
-            out.k = 0.0f;
-        }
-    } else if constexpr (P::cell_poly) {
-        if (b != cc.base) {
-            cc.base = b;
-            const V v0 = P::load(a.grid, b), v1 = P::load(a.grid, b + 1u);
-            const V v2 = P::load(a.grid, b + g.sy), v3 = P::load(a.grid, b + g.sy + 1u);
-            const V v4 = P::load(a.grid, b + g.sx), v5 = P::load(a.grid, b + g.sx + 1u);
-            const V v6 = P::load(a.grid, b + g.sx + g.sy), v7 = P::load(a.grid, b + g.sx + g.sy + 1u);
-            poly_coeffs<R>(cc.t[0], v0.x, v1.x, v2.x, v3.x, v4.x, v5.x, v6.x, v7.x);
-            poly_coeffs<R>(cc.t[1], v0.y, v1.y, v2.y, v3.y, v4.y, v5.y, v6.y, v7.y);
-            poly_coeffs<R>(cc.t[2], v0.z, v1.z, v2.z, v3.z, v4.z, v5.z, v6.z, v7.z);
-            poly_coeffs<R>(cc.t[3], v0.w, v1.w, v2.w, v3.w, v4.w, v5.w, v6.w, v7.w);
-            if constexpr (IB == IB_SUBCRITICAL) {
-                poly_coeffs<R>(cc.t[4 % (IB ? 5 : 4)], corner_x2(v0.x), corner_x2(v1.x), corner_x2(v2.x),
-                               corner_x2(v3.x), corner_x2(v4.x), corner_x2(v5.x), corner_x2(v6.x), corner_x2(v7.x));
-            } else if constexpr (IB == IB_GENERAL) {
-                poly_coeffs<R>(cc.t[4 % (IB ? 5 : 4)], corner_kappa<P>(a, v0.x), corner_kappa<P>(a, v1.x),
-                               corner_kappa<P>(a, v2.x), corner_kappa<P>(a, v3.x), corner_kappa<P>(a, v4.x),
-                               corner_kappa<P>(a, v5.x), corner_kappa<P>(a, v6.x), corner_kappa<P>(a, v7.x));
-            }
-        }
-        out.n1 = poly_eval<R>(cc.t[0], fx, fy, fz);
-        out.g0 = poly_eval<R>(cc.t[1], fx, fy, fz);
-        out.g1 = poly_eval<R>(cc.t[2], fx, fy, fz);
-        out.g2 = poly_eval<R>(cc.t[3], fx, fy, fz);
-        if constexpr (IB == IB_SUBCRITICAL) {
-            out.k = poly_eval<R>(cc.t[4 % (IB ? 5 : 4)], fx, fy, fz);   // cl_lo / ope2^2 is in tau_scale
-        } else if constexpr (IB == IB_GENERAL) {
-            out.k = poly_eval<R>(cc.t[4 % (IB ? 5 : 4)], fx, fy, fz);
-        } else {
-            out.k = R(0);
-        }
-    } else {
-        V c[8];
-        if constexpr (P::cell_cache) {
-            if (b != cc.base) {
-                cc.base = b;
-                cc.c[0] = P::load(a.grid, b);
-                cc.c[1] = P::load(a.grid, b + 1u);
-                cc.c[2] = P::load(a.grid, b + g.sy);
-                cc.c[3] = P::load(a.grid, b + g.sy + 1u);
-                cc.c[4] = P::load(a.grid, b + g.sx);
-                cc.c[5] = P::load(a.grid, b + g.sx + 1u);
-                cc.c[6] = P::load(a.grid, b + g.sx + g.sy);
-                cc.c[7] = P::load(a.grid, b + g.sx + g.sy + 1u);
-            }
-    #pragma unroll
-            for (int i = 0; i < 8; ++i) c[i] = cc.c[i];
-        } else {
-            c[0] = P::load(a.grid, b);
-            c[1] = P::load(a.grid, b + 1u);
-            c[2] = P::load(a.grid, b + g.sy);
-            c[3] = P::load(a.grid, b + g.sy + 1u);
-            c[4] = P::load(a.grid, b + g.sx);
-            c[5] = P::load(a.grid, b + g.sx + 1u);
-            c[6] = P::load(a.grid, b + g.sx + g.sy);
-            c[7] = P::load(a.grid, b + g.sx + g.sy + 1u);
-        }
-        const R ex = R(1) - fx, ey = R(1) - fy, ez = R(1) - fz;
-        const R w00 = ex * ey, w01 = ex * fy, w10 = fx * ey, w11 = fx * fy;
-        const R w[8] = {w00 * ez, w00 * fz, w01 * ez, w01 * fz, w10 * ez, w10 * fz, w11 * ez, w11 * fz};
-        R q = R(0), g0 = R(0), g1 = R(0), g2 = R(0);
-    #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            q += c[i].x * w[i];
-            g0 += c[i].y * w[i];
-            g1 += c[i].z * w[i];
-            g2 += c[i].w * w[i];
-        }
-        out.n1 = q;
-        out.g0 = g0;
-        out.g1 = g1;
-        out.g2 = g2;
-        if constexpr (IB == IB_SUBCRITICAL) {
-            R k = R(0);
-    #pragma unroll
-            for (int i = 0; i < 8; ++i) k += w[i] * corner_x2(c[i].x);
-            out.k = k;   // cl_lo / ope2^2 is in tau_scale
-        } else if constexpr (IB == IB_GENERAL) {
-            R k = R(0);
-    #pragma unroll
-            for (int i = 0; i < 8; ++i) k += w[i] * corner_kappa<P>(a, c[i].x);
-            out.k = k;
-        } else {
-            out.k = R(0);
+            R k[8];
+            poly_coeffs<R>(k, corner_kappa<P>(a, v0.x), corner_kappa<P>(a, v1.x), corner_kappa<P>(a, v2.x),
+                           corner_kappa<P>(a, v3.x), corner_kappa<P>(a, v4.x), corner_kappa<P>(a, v5.x),
+                           corner_kappa<P>(a, v6.x), corner_kappa<P>(a, v7.x));
+            kappa_store(k);
         }
     }
+    out.n1 = poly_eval<R>(cc.t[0], fx, fy, fz);
+    out.g0 = poly_eval<R>(cc.t[1], fx, fy, fz);
+    out.g1 = poly_eval<R>(cc.t[2], fx, fy, fz);
+    out.g2 = poly_eval<R>(cc.t[3], fx, fy, fz);
+    if constexpr (IB != IB_OFF) out.k = kappa_eval(fx, fy, fz);   // sub-critical: cl_lo / ope2^2 is in tau_scale
+    else out.k = R(0);
 }
 
 // One step of length phi (in steps; phi = 1 except for a step cut at a grid
@@ -570,9 +498,9 @@ __device__ __forceinline__ void rkn_step(const TraceArgs& a, Ray<P>& r, Cache& c
 __device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
 
 // sample at (hx + lx, hyz + lyz)
-template <int IB, int MODE, int NK>
+template <int IB, int MODE>
 __device__ __forceinline__ void sample_f2(const TraceArgs& a, float hx, float lx, float2 hyz, float2 lyz,
-                                          Sample<PolF32>& out, CellPolyF2<NK>& cc) {
+                                          Sample<PolF32>& out, CellPolyF2& cc) {
     const GridGeo& g = a.geo;
     float px = hx + lx;
     float2 pyz = __fadd2_rn(hyz, lyz);
@@ -639,8 +567,8 @@ __device__ __forceinline__ void kahan2_fma(float2& s, float2& c, float2 a, float
 // UNIT: phi is 1 (every step but a cut one); the multiplications by phi are
 // left out, which gives bitwise the results of the general form at phi = 1
 // (fma(1, a, b) rounds as a + b).
-template <int IB, int MODE, bool UNIT, int NK>
-__device__ __forceinline__ void rkn_step_f2(const TraceArgs& a, Ray<PolF32>& r, CellPolyF2<NK>& cc, float phi) {
+template <int IB, int MODE, bool UNIT>
+__device__ __forceinline__ void rkn_step_f2(const TraceArgs& a, Ray<PolF32>& r, CellPolyF2& cc, float phi) {
     if constexpr (UNIT) phi = 1.0f;
     auto mphi = [&](float x) { return UNIT ? x : __fmul_rn(phi, x); };
     auto mphi2 = [&](float2 x) { return UNIT ? x : __fmul2_rn(bc2(phi), x); };
@@ -812,8 +740,8 @@ __device__ __forceinline__ void rk4_step(const TraceArgs& a, Ray<P>& r, Cache& c
 
 // The RK4 step in the paired FP32 form (y and z components as register
 // pairs), every rounding explicit.
-template <int IB, int MODE, bool UNIT, int NK>
-__device__ __forceinline__ void rk4_step_f2(const TraceArgs& a, Ray<PolF32>& r, CellPolyF2<NK>& cc, float phi) {
+template <int IB, int MODE, bool UNIT>
+__device__ __forceinline__ void rk4_step_f2(const TraceArgs& a, Ray<PolF32>& r, CellPolyF2& cc, float phi) {
     if constexpr (UNIT) phi = 1.0f;
     auto mphi = [&](float x) { return UNIT ? x : __fmul_rn(phi, x); };
     auto mphi2 = [&](float2 x) { return UNIT ? x : __fmul2_rn(bc2(phi), x); };
@@ -896,20 +824,16 @@ __device__ __forceinline__ void rk4_step_f2(const TraceArgs& a, Ray<PolF32>& r, 
     if constexpr (IB != IB_OFF) r.tau.add(mphi(kq));
 }
 
-// One step: the paired FP32 form with the paired cell cache, the generic form
-// otherwise; RKN unless INTEG selects RK4.
+// One step: the paired form in FP32, the generic form in FP64; RKN unless
+// INTEG selects RK4.
 template <class P, int IB, int MODE, bool UNIT = false, int INTEG = INTEG_RKN, class Cache>
 __device__ __forceinline__ void step_any(const TraceArgs& a, Ray<P>& r, Cache& cc, typename P::R phi) {
-    if constexpr (INTEG == INTEG_RK4) {
-        if constexpr (IsPairedCache<Cache>::value && SLOTH_PAIRED_STEP) {
-            rk4_step_f2<IB, MODE, UNIT>(a, r, cc, phi);
-        } else {
-            rk4_step<P, IB, MODE>(a, r, cc, phi);
-        }
-    } else if constexpr (IsPairedCache<Cache>::value && SLOTH_PAIRED_STEP) {
-        rkn_step_f2<IB, MODE, UNIT>(a, r, cc, phi);
+    if constexpr (sizeof(typename P::R) == 4) {
+        if constexpr (INTEG == INTEG_RK4) rk4_step_f2<IB, MODE, UNIT>(a, r, cc, phi);
+        else rkn_step_f2<IB, MODE, UNIT>(a, r, cc, phi);
     } else {
-        rkn_step<P, IB, MODE>(a, r, cc, phi);
+        if constexpr (INTEG == INTEG_RK4) rk4_step<P, IB, MODE>(a, r, cc, phi);
+        else rkn_step<P, IB, MODE>(a, r, cc, phi);
     }
 }
 
@@ -1257,13 +1181,16 @@ __device__ __forceinline__ void trace_warp(const TraceArgs& a, Queue& q, Cache& 
     }
 }
 
-// Register cache of the last cell: polynomial coefficients or corners.
-template <class P, int IB>
-using CellCacheFor = typename std::conditional<
-    P::cell_poly,
-    typename std::conditional<std::is_same<typename P::R, float>::value && SLOTH_PAIRED_F32,
-                              CellPolyF2<(IB != IB_OFF) ? 5 : 4>, CellPoly<P, (IB != IB_OFF) ? 5 : 4>>::type,
-    CellCache<P>>::type;
+// The cell cache of a precision.
+template <class P>
+using CellCacheFor = typename std::conditional<sizeof(typename P::R) == 4, CellPolyF2, CellPolyD>::type;
+
+// One-warp CTAs per SM: FP32 at 128 registers; FP64 at 168, which holds the
+// polynomials without spilling (256^3 / 4e5 rays: 4.53 ms, against 5.33 ms
+// at 128 registers and 16 warps with 330 B of spill, 4.61 at 10 warps, 4.98 at 8).
+template <class P, int INTEG> constexpr int trace_min_blocks() {
+    return sizeof(typename P::R) == 4 ? SLOTH_TRACE_MIN_BLOCKS : (INTEG == INTEG_RK4 ? 8 : 12);
+}
 
 // Sum of `v` over the warp, added to *dst by one lane.
 __device__ __forceinline__ void warp_add(unsigned long long v, unsigned long long* dst) {
