@@ -52,9 +52,10 @@ def _device_rays(r) -> torch.Tensor:
         t = torch.from_numpy(np.ascontiguousarray(r))
     if t.dtype not in (torch.float32, torch.float64):
         t = t.to(torch.float64)
+    t = t.contiguous()
     if t.device.type != "cuda":
-        t = t.to(dev)
-    return t.contiguous()
+        t = runtime.upload(t, torch.empty(t.shape, dtype=t.dtype, device=dev))
+    return t
 
 
 def run_optics(rays, ops: Sequence[Op] = (), *, weights=None, pos_scale: float = 1.0,
@@ -122,7 +123,7 @@ def mm_to_m(r):
 
 def _apply(r, ops):
     out, _, _ = run_optics(r, ops, want_rays=True)
-    return out.cpu().numpy()
+    return runtime.download(out)
 
 
 def _reject_in_place(r, ops):
@@ -254,7 +255,7 @@ class Diagnostic:
             return self._rf_in.cpu().numpy()
         if self._rf_cache is None:
             out, _, _ = run_optics(self._rf_in, self._ops, pos_scale=1e3, want_rays=True)
-            self._rf_cache = out.cpu().numpy()
+            self._rf_cache = runtime.download(out)
         return self._rf_cache
 
     @rf.setter
@@ -287,7 +288,7 @@ class Diagnostic:
             src, ops, scale = self._rf_in, self._ops, 1e3
         _, _, H = run_optics(src, ops, weights=self._weights_dev, pos_scale=scale, ccd_half=ccd,
                              hist=(nx, ny, xr, yr))
-        self.H = H.cpu().numpy()
+        self.H = runtime.download(H)
         self.xedges = np.linspace(xr[0], xr[1], nx + 1)
         self.yedges = np.linspace(yr[0], yr[1], ny + 1)
         if clear_mem:

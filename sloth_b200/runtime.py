@@ -82,6 +82,38 @@ class DeviceGrid:
         return tuple(o + h * (k - 1) for o, h, k in zip(self.origin, self.spacing, self.n))
 
 
+_STAGE_BYTES = 8 << 20
+
+
+def upload(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
+    """Copy the CPU tensor src into the CUDA tensor dst (same shape and dtype,
+    both contiguous) on the current stream. Pinned memory is copied as it is,
+    without waiting. Pageable memory goes through pinned pieces that the host's threads
+    fill while the previous piece is copied (the driver's own staging fills
+    them with one thread: 67 MB in 5.6 ms); src may be changed once this returns."""
+    if src.nbytes <= _STAGE_BYTES // 8 or src.is_pinned():
+        return dst.copy_(src, non_blocking=True)
+    s, d = src.reshape(-1), dst.view(-1)
+    m = _STAGE_BYTES // src.element_size()
+    for a in range(0, s.numel(), m):
+        # the caching host allocator reuses a piece once its copy is done
+        piece = torch.empty(min(m, s.numel() - a), dtype=s.dtype, pin_memory=True)
+        piece.copy_(s[a:a + m])
+        d[a:a + m].copy_(piece, non_blocking=True)
+    return dst
+
+
+def download(t: torch.Tensor) -> np.ndarray:
+    """The CUDA tensor t as a numpy array (in pinned memory when it is large,
+    as trace_to_host's results are: 71 MB in 1.4 ms against 30 ms into pageable memory)."""
+    if t.nbytes <= _STAGE_BYTES // 8:
+        return t.cpu().numpy()
+    h = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
+    h.copy_(t, non_blocking=True)
+    torch.cuda.current_stream(t.device).synchronize()
+    return h.numpy()
+
+
 def _from_order_key(key: int) -> float:
     """The double of an order key of sloth_grid_pack_range (as int64)."""
     b = key & 0xFFFFFFFFFFFFFFFF
@@ -111,9 +143,9 @@ def pack_grid(ne, origin, spacing, omega, *, precision="f32", device=None, strea
         ne = ne.to(torch.float32)
     if ne.dim() != 3:
         raise ValueError("ne must be a 3-D (nx, ny, nz) array")
-    if ne.device.type != "cuda":
-        ne = ne.to(dev, non_blocking=True)
     ne = ne.contiguous()
+    if ne.device.type != "cuda":
+        ne = upload(ne, torch.empty(ne.shape, dtype=ne.dtype, device=dev))
     n = tuple(int(k) for k in ne.shape)
     desc = capi.grid_desc(n, origin, spacing)
     rb = 4 if precision == "f32" else 8
@@ -417,7 +449,10 @@ def trace_to_host(grid: DeviceGrid, rays, sched: Schedule, *, want: dict, chunk_
                 st = torch.empty((6, m), dtype=src.dtype, device=dev)
                 stage[li] = st
             for r in range(6):
-                st[r].copy_(src[r, a:b], non_blocking=True)
+                if src.device.type == "cuda":
+                    st[r].copy_(src[r, a:b], non_blocking=True)
+                else:
+                    upload(src[r, a:b], st[r])
             rc = st if src.dtype == dtype else st.to(dtype)
             o = trace(grid, rc, sched, stream=lane, workspace=_lane_workspace(m, dev, li), outputs=outs[li],
                       want_state="state" in want, want_phase="phase" in want, want_amp="amp" in want,
