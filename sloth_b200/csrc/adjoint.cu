@@ -43,23 +43,22 @@
 
 namespace sloth {
 
-constexpr int kAdjThreads = 256;
+// One-warp CTAs for the forward and the backward: a finished warp's place is
+// taken at once, and few rays spread over all SMs.
 // The backward's recompute of a checkpoint segment records where each stage
 // of each step sampled the field (its cell and in-cell coordinates), and the
-// step adjoints linearise there. Stages 1 and 2's in-cell coordinates go to
+// step adjoints linearise there. Five of a step's nine in-cell coordinates go to
 // shared memory, [step][word][thread] so that a warp's accesses are
-// consecutive (5 words per step); the three cells and the other in-cell
-// coordinates stay in a per-thread array. 128 threads per CTA: a 20-step
-// segment takes 51 KB of shared memory in FP32, so four CTAs share an SM
-// (16 warps; the kernel is latency-bound).
-constexpr int kAdjBwdThreads = 128;
+// consecutive; the three cells and the other coordinates stay in a per-thread
+// array. A 20-step segment takes 12.8 KB of shared memory per warp in FP32, so 16
+// warps share an SM (the kernel is latency-bound).
+constexpr int kAdjThreads = 32;
 constexpr int kAdjStateWords = 5;
-// Two FP32 builds of the backward: four CTAs per SM (128 registers) when
-// four segment buffers fit an SM's shared memory (on B200, 228 KB per SM and
-// 1 KB reserved per CTA: checkpoints at most every 21 steps), three (152
-// registers) otherwise. FP64 runs one CTA per SM.
-// The FP32 forward fits three 256-thread CTAs per SM (80 registers) without spilling.
-template <class P> constexpr int adj_fwd_min_blocks() { return sizeof(typename P::R) == 4 ? 3 : 1; }
+// Two FP32 builds of the backward: 16 warps per SM (128 registers) when as
+// many segment buffers fit an SM's shared memory (on B200, 228 KB per SM and
+// 1 KB reserved per CTA: checkpoints at most every 20 steps), 12 (168
+// registers) otherwise. FP64 runs 8. The FP32 forward runs 24 (80 registers).
+template <class P> constexpr int adj_fwd_min_blocks() { return sizeof(typename P::R) == 4 ? 24 : 12; }
 constexpr int kMaxCkptEvery = 32;
 constexpr int kMaxTaps = 65;          // 2 * 4 * sigma + 1 pixels at sigma <= 8
 
@@ -72,6 +71,7 @@ struct ImageArgs {
     double origin[3], w_of_v[3], inv_h[3];
     double S[3];                 // -(dtau/h)^2 / 2
     float Sf[3];                 // S rounded to FP32 once on the host (the FP32 kernels' copy)
+    float S4f[3], S2f[3], S6f[3];   // Sf/4, Sf/2 and fl(1/6)*Sf: the FP32 step's coefficients
     int n_steps, ckpt_every, n_seg;
     int axis, t1, t2;
     double plane;                // detector plane (cells along axis)
@@ -171,28 +171,17 @@ struct GradCell {
 // Cell and in-cell coordinates of the point hi + lo (the tracer's split: the
 // cell from the rounded sum, the fractions from (hi - i) + lo). False when
 // the point is outside the grid (fill 0).
-template <class P, bool INTERIOR = false>
+template <class P>
 __device__ __forceinline__ bool locate(const GridGeo& g, const typename P::R (&hi)[3],
                                        const typename P::R (&lo)[3], unsigned& base, typename P::R (&f)[3]) {
     using R = typename P::R;
     R p[3];
 #pragma unroll
     for (int x = 0; x < 3; ++x) p[x] = hi[x] + lo[x];
-    int ix, iy, iz;
-    if constexpr (!INTERIOR) {
-        const bool in = (p[0] >= R(0)) & (p[0] <= lim_of<R>(g, 0)) & (p[1] >= R(0)) &
-                        (p[1] <= lim_of<R>(g, 1)) & (p[2] >= R(0)) & (p[2] <= lim_of<R>(g, 2));
-        if (!in) return false;
-        ix = min((int)p[0], g.n[0] - 2);
-        iy = min((int)p[1], g.n[1] - 2);
-        iz = min((int)p[2], g.n[2] - 2);
-    } else {
-        // a point of an interior step: inside by construction; one unsigned
-        // min per axis keeps the index in the grid all the same
-        ix = (int)min((unsigned)(int)p[0], (unsigned)(g.n[0] - 2));
-        iy = (int)min((unsigned)(int)p[1], (unsigned)(g.n[1] - 2));
-        iz = (int)min((unsigned)(int)p[2], (unsigned)(g.n[2] - 2));
-    }
+    const bool in = (p[0] >= R(0)) & (p[0] <= lim_of<R>(g, 0)) & (p[1] >= R(0)) & (p[1] <= lim_of<R>(g, 1)) &
+                    (p[2] >= R(0)) & (p[2] <= lim_of<R>(g, 2));
+    if (!in) return false;
+    const int ix = min((int)p[0], g.n[0] - 2), iy = min((int)p[1], g.n[1] - 2), iz = min((int)p[2], g.n[2] - 2);
     f[0] = (hi[0] - (R)ix) + lo[0];
     f[1] = (hi[1] - (R)iy) + lo[1];
     f[2] = (hi[2] - (R)iz) + lo[2];
@@ -205,7 +194,8 @@ __device__ __forceinline__ bool locate(const GridGeo& g, const typename P::R (&h
 // sm_100's paired FP32 instructions (q is carried along at no cost).
 struct GradCellF2 {
     unsigned base;
-    float2 t[2][8];
+    float t0[8];      // dq/du
+    float2 t1[8];     // (dq/dv, dq/dw)
 };
 
 __device__ __forceinline__ void load_cell_f2(const ImageArgs& a, unsigned b, GradCellF2& cc) {
@@ -217,13 +207,10 @@ __device__ __forceinline__ void load_cell_f2(const ImageArgs& a, unsigned b, Gra
     const float4 v2 = __ldg(gp + b + g.sy), v3 = __ldg(gp + b + g.sy + 1u);
     const float4 v4 = __ldg(gp + b + g.sx), v5 = __ldg(gp + b + g.sx + 1u);
     const float4 v6 = __ldg(gp + b + g.sx + g.sy), v7 = __ldg(gp + b + g.sx + g.sy + 1u);
-#define SLOTH_LO(v) make_float2(v.x, v.y)
 #define SLOTH_HI(v) make_float2(v.z, v.w)
-    poly_coeffs2(cc.t[0], SLOTH_LO(v0), SLOTH_LO(v1), SLOTH_LO(v2), SLOTH_LO(v3), SLOTH_LO(v4), SLOTH_LO(v5),
-                 SLOTH_LO(v6), SLOTH_LO(v7));
-    poly_coeffs2(cc.t[1], SLOTH_HI(v0), SLOTH_HI(v1), SLOTH_HI(v2), SLOTH_HI(v3), SLOTH_HI(v4), SLOTH_HI(v5),
+    poly_coeffs<float>(cc.t0, v0.y, v1.y, v2.y, v3.y, v4.y, v5.y, v6.y, v7.y);
+    poly_coeffs2(cc.t1, SLOTH_HI(v0), SLOTH_HI(v1), SLOTH_HI(v2), SLOTH_HI(v3), SLOTH_HI(v4), SLOTH_HI(v5),
                  SLOTH_HI(v6), SLOTH_HI(v7));
-#undef SLOTH_LO
 #undef SLOTH_HI
 }
 
@@ -254,15 +241,15 @@ struct StageRec {
     typename P::R f[3];
 };
 
-// Acceleration S * grad(q) at hi + lo (zero outside); with rec, where it
+// FP64: acceleration S * grad(q) at hi + lo (zero outside); with rec, where it
 // sampled.
-template <class P, bool INTERIOR, class Cell>
+template <class P>
 __device__ __forceinline__ void accel(const ImageArgs& a, const typename P::R (&hi)[3], const typename P::R (&lo)[3],
-                                      typename P::R (&A)[3], Cell& cc, StageRec<P>* rec = nullptr) {
+                                      typename P::R (&A)[3], GradCell<P>& cc, StageRec<P>* rec) {
     using R = typename P::R;
     unsigned b;
     R f[3];
-    if (!locate<P, INTERIOR>(a.geo, hi, lo, b, f)) {
+    if (!locate<P>(a.geo, hi, lo, b, f)) {
         A[0] = A[1] = A[2] = R(0);
         if (rec) {
             rec->b = kNone;
@@ -276,26 +263,101 @@ __device__ __forceinline__ void accel(const ImageArgs& a, const typename P::R (&
         rec->f[1] = f[1];
         rec->f[2] = f[2];
     }
-    if constexpr (std::is_same<Cell, GradCellF2>::value) {
-        load_cell_f2(a, b, cc);
-        const float2 fx = make_float2(f[0], f[0]), fy = make_float2(f[1], f[1]), fz = make_float2(f[2], f[2]);
-        const float2 r0 = poly_eval2(cc.t[0], fx, fy, fz), r1 = poly_eval2(cc.t[1], fx, fy, fz);
-        A[0] = img_S<R>(a, 0) * r0.y;
-        A[1] = img_S<R>(a, 1) * r1.x;
-        A[2] = img_S<R>(a, 2) * r1.y;
-    } else {
-        load_cell<P>(a, b, cc);
+    load_cell<P>(a, b, cc);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) A[k] = img_S<R>(a, k) * poly_eval<R>(cc.t[k], f[0], f[1], f[2]);
+    for (int k = 0; k < 3; ++k) A[k] = a.S[k] * poly_eval<R>(cc.t[k], f[0], f[1], f[2]);
+}
+
+// FP32: the gradient at (hx + lx, hyz + lyz), y and z as a pair (zero outside);
+// with rec, where it sampled.
+template <bool INTERIOR>
+__device__ __forceinline__ void gradient_f2(const ImageArgs& a, float hx, float lx, float2 hyz, float2 lyz, float& Gx,
+                                            float2& Gyz, GradCellF2& cc, StageRec<PolF32>* rec) {
+    const GridGeo& g = a.geo;
+    const float px = hx + lx;
+    const float2 pyz = __fadd2_rn(hyz, lyz);
+    int ix, iy, iz;
+    if constexpr (!INTERIOR) {
+        const bool in = (px >= 0.0f) & (px <= g.limf[0]) & (pyz.x >= 0.0f) & (pyz.x <= g.limf[1]) &
+                        (pyz.y >= 0.0f) & (pyz.y <= g.limf[2]);
+        if (!in) {
+            Gx = 0.0f;
+            Gyz = make_float2(0.0f, 0.0f);
+            if (rec) {
+                rec->b = kNone;
+                rec->f[0] = rec->f[1] = rec->f[2] = 0.0f;
+            }
+            return;
+        }
+        ix = min((int)px, g.n[0] - 2);
+        iy = min((int)pyz.x, g.n[1] - 2);
+        iz = min((int)pyz.y, g.n[2] - 2);
+    } else {
+        // a point of an interior step: inside by construction; one unsigned
+        // min per axis keeps the index in the grid all the same
+        ix = (int)min((unsigned)(int)px, (unsigned)(g.n[0] - 2));
+        iy = (int)min((unsigned)(int)pyz.x, (unsigned)(g.n[1] - 2));
+        iz = (int)min((unsigned)(int)pyz.y, (unsigned)(g.n[2] - 2));
     }
+    const float fx = (hx - (float)ix) + lx;
+    const float2 fyz = __fadd2_rn(__fadd2_rn(hyz, make_float2(-(float)iy, -(float)iz)), lyz);
+    const unsigned b = (unsigned)ix * g.sx + (unsigned)iy * g.sy + (unsigned)iz;
+    if (rec) {
+        rec->b = b;
+        rec->f[0] = fx;
+        rec->f[1] = fyz.x;
+        rec->f[2] = fyz.y;
+    }
+    load_cell_f2(a, b, cc);
+    Gx = poly_eval<float>(cc.t0, fx, fyz.x, fyz.y);
+    Gyz = poly_eval2(cc.t1, bc2(fx), bc2(fyz.x), bc2(fyz.y));
 }
 
 // One step (the tracer's Runge-Kutta-Nystrom step with phi = 1, without
 // phase and depth):
 //   p' = p + w + (A1 + 2 A2)/6,  w' = w + (A1 + 4 A2 + A3)/6,
 //   stages at p, p + w/2 + A1/8, p + w + A2/2.
-template <class P, bool INTERIOR = false, class Cell>
-__device__ __forceinline__ void model_step(const ImageArgs& a, MState<P>& r, Cell& cc, StageRec<P>* rec = nullptr) {
+// INTERIOR (FP32): the step's points are known to lie inside the grid, bitwise
+// the same step. The FP32 step is the tracer's paired one: S in the coefficients,
+// y and z as register pairs, every rounding explicit, so that the forward's and the
+// recompute's steps agree bit for bit.
+template <bool INTERIOR>
+__device__ __forceinline__ void model_step(const ImageArgs& a, MState<PolF32>& r, GradCellF2& cc,
+                                           StageRec<PolF32>* rec = nullptr) {
+    const float phx = r.p[0].s, plx = r.p[0].c, wex = __fadd_rn(r.w[0].s, r.w[0].c);
+    const float2 phyz = make_float2(r.p[1].s, r.p[2].s), plyz = make_float2(r.p[1].c, r.p[2].c);
+    const float2 whi = make_float2(r.w[1].s, r.w[2].s), wlo = make_float2(r.w[1].c, r.w[2].c);
+    const float2 weyz = __fadd2_rn(whi, wlo);
+    const float2 S6yz = make_float2(a.S6f[1], a.S6f[2]);
+    float Gx;
+    float2 Gyz;
+    gradient_f2<INTERIOR>(a, phx, plx, phyz, plyz, Gx, Gyz, cc, rec);
+    float gAx = Gx, gWx = Gx;                   // g1 + 2 g2 and g1 + 4 g2 + g3
+    float2 gAyz = Gyz, gWyz = Gyz;
+    float stx = __fmaf_rn(0.5f, __fmaf_rn(a.S4f[0], Gx, wex), plx);       // p + (w + S/4 G1)/2
+    float2 styz = __ffma2_rn(bc2(0.5f), __ffma2_rn(make_float2(a.S4f[1], a.S4f[2]), Gyz, weyz), plyz);
+    gradient_f2<INTERIOR>(a, phx, stx, phyz, styz, Gx, Gyz, cc, rec ? rec + 1 : nullptr);
+    gAx = __fmaf_rn(2.0f, Gx, gAx);
+    gAyz = __ffma2_rn(bc2(2.0f), Gyz, gAyz);
+    gWx = __fmaf_rn(4.0f, Gx, gWx);
+    gWyz = __ffma2_rn(bc2(4.0f), Gyz, gWyz);
+    stx = __fadd_rn(plx, __fmaf_rn(a.S2f[0], Gx, wex));                   // p + w + S/2 G2
+    styz = __fadd2_rn(plyz, __ffma2_rn(make_float2(a.S2f[1], a.S2f[2]), Gyz, weyz));
+    gradient_f2<INTERIOR>(a, phx, stx, phyz, styz, Gx, Gyz, cc, rec ? rec + 2 : nullptr);
+    gWx = __fadd_rn(gWx, Gx);
+    gWyz = __fadd2_rn(gWyz, Gyz);
+    r.p[0].add(__fadd_rn(r.w[0].hi(), __fmaf_rn(a.S6f[0], gAx, r.w[0].lo())));
+    r.w[0].add_fma(a.S6f[0], gWx);
+    float2 ps = phyz, pc = plyz, ws = whi, wc = wlo;
+    kahan2(ps, pc, __fadd2_rn(whi, __ffma2_rn(S6yz, gAyz, wlo)));
+    kahan2_fma(ws, wc, S6yz, gWyz);
+    r.p[1].s = ps.x; r.p[2].s = ps.y; r.p[1].c = pc.x; r.p[2].c = pc.y;
+    r.w[1].s = ws.x; r.w[2].s = ws.y; r.w[1].c = wc.x; r.w[2].c = wc.y;
+}
+
+template <bool INTERIOR, class P>
+__device__ __forceinline__ void model_step(const ImageArgs& a, MState<P>& r, GradCell<P>& cc,
+                                           StageRec<P>* rec = nullptr) {
     using R = typename P::R;
     R ph[3], pl[3], we[3], st[3], A1[3], A2[3], A3[3];
 #pragma unroll
@@ -304,13 +366,13 @@ __device__ __forceinline__ void model_step(const ImageArgs& a, MState<P>& r, Cel
         pl[x] = r.p[x].lo();
         we[x] = r.w[x].val();
     }
-    accel<P, INTERIOR>(a, ph, pl, A1, cc, rec);
+    accel<P>(a, ph, pl, A1, cc, rec);
 #pragma unroll
     for (int x = 0; x < 3; ++x) st[x] = pl[x] + (R(0.5) * we[x] + R(0.125) * A1[x]);
-    accel<P, INTERIOR>(a, ph, st, A2, cc, rec ? rec + 1 : nullptr);
+    accel<P>(a, ph, st, A2, cc, rec ? rec + 1 : nullptr);
 #pragma unroll
     for (int x = 0; x < 3; ++x) st[x] = pl[x] + (we[x] + R(0.5) * A2[x]);
-    accel<P, INTERIOR>(a, ph, st, A3, cc, rec ? rec + 2 : nullptr);
+    accel<P>(a, ph, st, A3, cc, rec ? rec + 2 : nullptr);
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
         const R sA = A1[x] + R(2) * A2[x];
@@ -448,13 +510,13 @@ __device__ __forceinline__ void stage_adjoint(const ImageArgs& a, const StageRec
     float gb[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) gb[k] = img_S<float>(a, k) * Abar[k];
-    // J^T gb. Channel 1 (dq/du) is the .y half of pair 0, channels 2 and 3 are pair 1.
-    const float2* t0 = cc.t[0];
-    const float2* t1 = cc.t[1];
-    const float u76 = fmaf(fx, t0[7].y, t0[6].y);
-    const float d1x = fmaf(fz, fmaf(fy, t0[7].y, t0[5].y), fmaf(fy, t0[4].y, t0[1].y));
-    const float d1y = fmaf(fz, u76, fmaf(fx, t0[4].y, t0[2].y));
-    const float d1z = fmaf(fy, u76, fmaf(fx, t0[5].y, t0[3].y));
+    // J^T gb. Channel 1 (dq/du) is t0, channels 2 and 3 are the pairs t1.
+    const float* t0 = cc.t0;
+    const float2* t1 = cc.t1;
+    const float u76 = fmaf(fx, t0[7], t0[6]);
+    const float d1x = fmaf(fz, fmaf(fy, t0[7], t0[5]), fmaf(fy, t0[4], t0[1]));
+    const float d1y = fmaf(fz, u76, fmaf(fx, t0[4], t0[2]));
+    const float d1z = fmaf(fy, u76, fmaf(fx, t0[5], t0[3]));
     const float2 v76 = __ffma2_rn(fx2, t1[7], t1[6]);
     const float2 d2x = __ffma2_rn(fz2, __ffma2_rn(fy2, t1[7], t1[5]), __ffma2_rn(fy2, t1[4], t1[1]));
     const float2 d2y = __ffma2_rn(fz2, v76, __ffma2_rn(fx2, t1[4], t1[2]));
@@ -627,54 +689,60 @@ __device__ __forceinline__ bool detector_point(const ImageArgs& a, const MState<
     return isfinite(pa) && isfinite(pb) && fabs(pa) < 1e9 && fabs(pb) < 1e9;
 }
 
-template <class P>
-__device__ __forceinline__ void splat(const ImageArgs& a, double pa, double pb) {
-    using R = typename P::R;
-    const int i0 = (int)floor(pa - a.radius) + 1;
-    const int j0 = (int)floor(pb - a.radius) + 1;
-    const R s = (R)a.sigma;
-    R gy[kMaxTaps];
-    for (int j = 0; j < a.taps; ++j) {
-        R dg;
-        gy[j] = splat_g<R>((R)((double)(j0 + j) - pb), s, dg);
+// The splats of a block of rays, formed in shared memory and added to the
+// image once per pixel and tile. Rays that are neighbours at entry overlap on the
+// detector; adding each ray's taps to the image directly (17 x 17 reductions per
+// ray at sigma = 2) serialises in L2: at 3e4 rays on 97 x 97 pixels that alone took
+// 90 us. The block's first ray that is left sets a kSplatTile x kSplatTile tile with its
+// window in the middle; the rays whose windows (clipped to the image) fit in it
+// leave their separable weights g(i - a) * norm (rows) and g(j - b) (columns) over
+// the tile in shared memory, splat_rays at a time, and pixel (r, c) = sum over rays
+// of row_weight(r) * column_weight(c), a small matrix product: four groups of 64
+// threads take a quarter of the rays each, a thread 4 x 4 pixels (two 16-byte
+// loads per 16 multiply-adds), and the groups' sums meet in shared memory. The next ray
+// left sets the next tile, kSplatRounds times at most; what is then left (rays
+// far apart, or windows larger than a tile) is splatted by its warp, one ray after
+// the other, its lanes on consecutive taps, so that a reduction covers whole rows of
+// the window.
+constexpr int kSplatRounds = 6;
+constexpr int kSplatMin = 8;                  // rays that are worth a tile
+constexpr int kSplatThreads = 256;
+constexpr int kSplatTile = 32;                // pixels per side of a block's tile
+constexpr int kSplatPitch = kSplatTile + 4;   // 16-byte rows
+template <class P> constexpr int splat_rays() { return sizeof(typename P::R) == 4 ? 64 : 32; }   // staged per round
+
+template <class R> struct Quad { R v[4]; };
+template <class R> __device__ __forceinline__ Quad<R> load_quad(const R* p) {
+    Quad<R> q;
+    if constexpr (sizeof(R) == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        q.v[0] = x.x; q.v[1] = x.y; q.v[2] = x.z; q.v[3] = x.w;
+    } else {
+        const double2 x = reinterpret_cast<const double2*>(p)[0], y = reinterpret_cast<const double2*>(p)[1];
+        q.v[0] = x.x; q.v[1] = x.y; q.v[2] = y.x; q.v[3] = y.y;
     }
-    R* img = reinterpret_cast<R*>(a.image);
-    for (int i = 0; i < a.taps; ++i) {
-        const int ii = i0 + i;
-        if (ii < 0 || ii >= a.npx[0]) continue;
-        R dg;
-        const R gx = splat_g<R>((R)((double)ii - pa), s, dg) * (R)a.norm;
-        if (gx == R(0)) continue;
-        for (int j = 0; j < a.taps; ++j) {
-            const int jj = j0 + j;
-            if (jj < 0 || jj >= a.npx[1] || gy[j] == R(0)) continue;
-            atomicAdd(img + (size_t)ii * a.npx[1] + jj, gx * gy[j]);
-        }
-    }
+    return q;
 }
 
-// A CTA's splats, formed in shared memory and added to the image once per
-// pixel. The rays of a CTA share their entry cell, so their windows overlap
-// on the detector; adding each ray's taps to the image directly (17 x 17
-// reductions per ray at sigma = 2) made the image's L2 atomics a third of the
-// forward's time. Here the CTA takes the box of its rays' windows (clipped to
-// the image). When a window fits in the kSplatTile x kSplatTile tile at the
-// box's low corner, the ray's separable weights g(i - a) * norm (rows) and
-// g(j - b) (columns) over the tile go to shared memory, kSplatRays rays at a
-// time, and every thread sums ray products for four pixels of the tile:
-// pixel (r, c) = sum over rays of row_weight(r) * column_weight(c), a small
-// matrix product. Windows that do not fit are splatted directly. Every thread
-// of the CTA calls this (it synchronises the CTA).
-constexpr int kSplatTile = 32;     // pixels per side of a CTA's tile
-constexpr int kSplatRays = 64;     // rays staged per round
-constexpr int kSplatPitch = kSplatTile + 1;   // shared row pitch (conflict-free stores and loads)
-
 template <class P>
-__device__ __forceinline__ void splat_block(const ImageArgs& a, bool has, double pa, double pb) {
+__global__ void __launch_bounds__(kSplatThreads) splat_kernel(const __grid_constant__ ImageArgs a) {
     using R = typename P::R;
-    __shared__ R s_row[kSplatRays * kSplatPitch], s_col[kSplatRays * kSplatPitch];
-    __shared__ int s_box[2];
-    const int t = threadIdx.x;
+    constexpr int kRays = splat_rays<P>(), kWarps = kSplatThreads / 32;
+    __shared__ __align__(16) R s_row[kRays * kSplatPitch], s_col[kRays * kSplatPitch];
+    __shared__ R s_tile[kSplatTile * kSplatTile];
+    __shared__ double s_a[kSplatThreads], s_b[kSplatThreads];
+    __shared__ int s_box[2], s_count[kWarps];
+    static_assert(kWarps * 2 * kMaxTaps <= kRays * kSplatPitch, "the warps' tap weights share s_row");
+    const int t = threadIdx.x, lane = t & 31;
+    const long long slot = (long long)blockIdx.x * kSplatThreads + t;
+    bool has = false;
+    double pa = 0.0, pb = 0.0;
+    if (slot < a.n) {
+        MState<P> r;
+        load_state<P>(a, a.n_seg, slot, r);
+        double tt, p[3], w[3];
+        has = detector_point<P>(a, r, pa, pb, tt, p, w);
+    }
     int i0 = 0, j0 = 0, r0 = 0, r1 = -1, c0 = 0, c1 = -1;
     if (has) {
         i0 = (int)floor(pa - a.radius) + 1;
@@ -684,52 +752,119 @@ __device__ __forceinline__ void splat_block(const ImageArgs& a, bool has, double
         c0 = max(j0, 0);
         c1 = min(j0 + a.taps - 1, a.npx[1] - 1);
     }
-    const bool in = r0 <= r1 && c0 <= c1;
-    if (t == 0) s_box[0] = s_box[1] = INT_MAX;
-    __syncthreads();
-    if (in) {
-        atomicMin(&s_box[0], r0);
-        atomicMin(&s_box[1], c0);
+    const R s = (R)a.sigma;
+    R* img = reinterpret_cast<R*>(a.image);
+    const int group = t >> 6, rb = 4 * ((t >> 3) & 7), cb = 4 * (t & 7), wid = t >> 5;
+    bool left_over = r0 <= r1 && c0 <= c1, direct = false;
+    for (int round = 0; round < kSplatRounds; ++round) {
+        // the first ray that is left sets the tile
+        const unsigned lmask = __ballot_sync(0xffffffffu, left_over);
+        if (lane == 0) s_count[wid] = lmask ? (t + __ffs(lmask) - 1) : INT_MAX;
+        __syncthreads();
+        int lead = INT_MAX;
+#pragma unroll
+        for (int k = 0; k < kWarps; ++k) lead = min(lead, s_count[k]);
+        if (lead == INT_MAX) break;        // the same in every thread
+        if (t == lead) {
+            s_box[0] = max((r0 + r1 + 1) / 2 - kSplatTile / 2, 0);
+            s_box[1] = max((c0 + c1 + 1) / 2 - kSplatTile / 2, 0);
+        }
+        __syncthreads();
+        const int br = s_box[0], bc = s_box[1];
+        const bool tiled = left_over && r0 >= br && r1 < br + kSplatTile && c0 >= bc && c1 < bc + kSplatTile;
+        // the tile's rays, compacted
+        const unsigned tmask = __ballot_sync(0xffffffffu, tiled);
+        if (lane == 0) s_count[wid] = __popc(tmask);
+        __syncthreads();
+        int before = 0, members = 0;
+#pragma unroll
+        for (int k = 0; k < kWarps; ++k) {
+            before += k < wid ? s_count[k] : 0;
+            members += s_count[k];
+        }
+        if (tiled) {
+            const int at = before + __popc(tmask & ((1u << lane) - 1u));
+            s_a[at] = pa;
+            s_b[at] = pb;
+        }
+        __syncthreads();
+        if (members < kSplatMin) {         // not worth a tile (none when the window is larger than it)
+            direct = direct || tiled || t == lead;
+            left_over = left_over && !direct;
+            continue;
+        }
+        left_over = left_over && !tiled;
+        R acc[4][4] = {};
+        for (int base = 0; base < members; base += kRays) {
+            // weights: this thread's share of 2 * kSplatTile per staged ray
+            constexpr int kShare = kSplatThreads / kRays;
+            const int u = t / kShare;
+            const bool mine = base + u < members;
+            const double qa = mine ? s_a[base + u] : 0.0, qb = mine ? s_b[base + u] : 0.0;
+            for (int k = t % kShare; k < kSplatTile; k += kShare) {
+                R dg;
+                const int ii = br + k, jj = bc + k;
+                const double di = (double)ii - qa, dj = (double)jj - qb;
+                s_row[u * kSplatPitch + k] =
+                    mine && fabs(di) < a.radius && ii < a.npx[0] ? splat_g<R>((R)di, s, dg) * (R)a.norm : R(0);
+                s_col[u * kSplatPitch + k] = mine && fabs(dj) < a.radius && jj < a.npx[1] ? splat_g<R>((R)dj, s, dg) : R(0);
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (int v = group * (kRays / 4); v < (group + 1) * (kRays / 4); ++v) {
+                const Quad<R> x = load_quad(s_row + v * kSplatPitch + rb), y = load_quad(s_col + v * kSplatPitch + cb);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] += x.v[i] * y.v[j];
+            }
+            __syncthreads();
+        }
+        for (int g = 0; g < 4; ++g) {
+            if (group == g) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        R& d = s_tile[(rb + i) * kSplatTile + cb + j];
+                        d = g ? d + acc[i][j] : acc[i][j];
+                    }
+            }
+            __syncthreads();
+        }
+        for (int k = t; k < kSplatTile * kSplatTile; k += kSplatThreads) {
+            const int ii = br + k / kSplatTile, jj = bc + k % kSplatTile;
+            const R v = s_tile[k];
+            if (v != R(0) && ii < a.npx[0] && jj < a.npx[1]) atomicAdd(img + (size_t)ii * a.npx[1] + jj, v);
+        }
     }
     __syncthreads();
-    const int br = s_box[0], bc = s_box[1];
-    const bool tiled = in && r1 < br + kSplatTile && c1 < bc + kSplatTile;
-    if (in && !tiled) splat<P>(a, pa, pb);
-    if (!__syncthreads_or(tiled)) return;
-    // this thread's four pixels: column c, rows r, r + 8, r + 16, r + 24
-    const int c = t & (kSplatTile - 1), rb = t >> 5;
-    static_assert(kAdjThreads == 256 && kSplatTile == 32, "four pixels per thread");
-    R acc[4] = {R(0), R(0), R(0), R(0)};
-    const R s = (R)a.sigma;
-    for (int base = 0; base < (int)blockDim.x; base += kSplatRays) {
-        if (t >= base && t < base + kSplatRays) {
-            R* rw = s_row + (t - base) * kSplatPitch;
-            R* cw = s_col + (t - base) * kSplatPitch;
-            for (int k = 0; k < kSplatTile; ++k) {
-                R g = R(0), dg;
-                const int ii = br + k;
-                if (tiled && ii >= r0 && ii <= r1) g = splat_g<R>((R)((double)ii - pa), s, dg) * (R)a.norm;
-                rw[k] = g;
-                R h = R(0);
-                const int jj = bc + k;
-                if (tiled && jj >= c0 && jj <= c1) h = splat_g<R>((R)((double)jj - pb), s, dg);
-                cw[k] = h;
+
+    unsigned left = __ballot_sync(0xffffffffu, left_over || direct);
+    if (left) {
+        R* gx = s_row + (t >> 5) * 2 * kMaxTaps;
+        R* gy = gx + kMaxTaps;
+        const float inv = 1.0f / (float)a.taps;
+        for (; left; left &= left - 1) {
+            const int src = __ffs(left) - 1;
+            const double qa = __shfl_sync(0xffffffffu, pa, src), qb = __shfl_sync(0xffffffffu, pb, src);
+            const int qi = __shfl_sync(0xffffffffu, i0, src), qj = __shfl_sync(0xffffffffu, j0, src);
+            __syncwarp();
+            for (int k = lane; k < a.taps; k += 32) {
+                R dg;
+                gx[k] = splat_g<R>((R)((double)(qi + k) - qa), s, dg) * (R)a.norm;
+                gy[k] = splat_g<R>((R)((double)(qj + k) - qb), s, dg);
+            }
+            __syncwarp();
+            for (int k = lane; k < a.taps * a.taps; k += 32) {
+                const int i = (int)(((float)k + 0.5f) * inv), j = k - i * a.taps;   // taps <= 65: exact
+                const int ii = qi + i, jj = qj + j;
+                if (ii >= 0 && ii < a.npx[0] && jj >= 0 && jj < a.npx[1]) {
+                    const R v = gx[i] * gy[j];
+                    if (v != R(0)) atomicAdd(img + (size_t)ii * a.npx[1] + jj, v);
+                }
             }
         }
-        __syncthreads();
-#pragma unroll 4
-        for (int u = 0; u < kSplatRays; ++u) {
-            const R h = s_col[u * kSplatPitch + c];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[q] += s_row[u * kSplatPitch + rb + 8 * q] * h;
-        }
-        __syncthreads();
-    }
-    R* img = reinterpret_cast<R*>(a.image);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int ii = br + rb + 8 * q, jj = bc + c;
-        if (acc[q] != R(0) && ii < a.npx[0] && jj < a.npx[1]) atomicAdd(img + (size_t)ii * a.npx[1] + jj, acc[q]);
     }
 }
 
@@ -856,60 +991,72 @@ __global__ void __launch_bounds__(256) accel_bound_kernel(const void* __restrict
 // ---------------------------------------------------------------------------
 // Kernels.
 // ---------------------------------------------------------------------------
+// One warp per CTA, one thread per ray: steps to the end, a checkpoint every
+// ckpt_every steps and the final state. The warp's rays run in step, so between
+// checkpoints (and for as many steps as every live ray's run allows) the steps
+// follow each other in a uniform loop. Bound by instruction issue (71 %, FMA pipe 64 %):
+// 128^3, 1e6 rays, 400 steps in 2.94 ms (1.33e11 ray-steps/s), 185 instructions a
+// ray-step; 3.26 ms and 235 before the paired step, the scalar dq/du polynomial and
+// this loop.
 template <class P>
 __global__ void __launch_bounds__(kAdjThreads, adj_fwd_min_blocks<P>()) image_forward_kernel(const __grid_constant__ ImageArgs a) {
     using R = typename P::R;
-    __shared__ unsigned long long s_steps;
-    if (threadIdx.x == 0) s_steps = 0;
-    __syncthreads();
-    const long long slot = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int t = 0;
-    bool has = false;     // the ray meets the detector plane at (pa, pb) pixels
-    double pa = 0.0, pb = 0.0;
-    if (slot < a.n) {
+    const long long slot = (long long)blockIdx.x * kAdjThreads + threadIdx.x;
+    bool active = slot < a.n;
+    MState<P> r;
+    if (active) {
         const unsigned id = a.perm[slot];
         const R* rays = reinterpret_cast<const R*>(a.rays);
-        MState<P> r;
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
             r.p[x].set(((double)rays[x * a.n + id] - a.origin[x]) * a.inv_h[x]);
             r.w[x].set((double)rays[(3 + x) * a.n + id] * a.w_of_v[x]);
         }
-        typename AdjTypes<P>::Cell cc;
-        cc.base = kNone;
-        const float B = load_accel_bound(a);
-        const bool fast = B <= (float)kInteriorAccel;
-        int run = 0, ck = 0, seg = 0;    // ck: steps to the next checkpoint
-        for (; t < a.n_steps; ++t) {
-            bool interior = false;
-            if (run > 0) {
-                // proven interior: inside, so not gone either
+    }
+    typename AdjTypes<P>::Cell cc;
+    cc.base = kNone;
+    const float B = load_accel_bound(a);
+    const bool fast = B <= (float)kInteriorAccel;
+    int t = 0, run = 0, ck = 0, seg = 0;    // run: steps ahead that are proven interior; ck: steps to the next checkpoint
+    while (__any_sync(0xffffffffu, active)) {
+        bool interior = false;
+        if (active) {
+            if (run > 0) {                  // inside, so not gone either
                 --run;
                 interior = true;
-            } else {
-                if (ray_gone_model<P>(a, r)) break;
-                if (fast && model_interior<P>(a, r)) {
-                    interior = true;
-                    run = model_interior_run<P>(a, r, B);
-                }
+            } else if (ray_gone_model<P>(a, r)) {
+                active = false;
+            } else if (fast && model_interior<P>(a, r)) {
+                interior = true;
+                run = model_interior_run<P>(a, r, B);
             }
-            if (ck == 0) {
-                store_state<P>(a, seg++, slot, r);
-                ck = a.ckpt_every;
-            }
-            --ck;
-            if (interior)
-                model_step<P, true>(a, r, cc);
-            else
-                model_step<P>(a, r, cc);
         }
+        if (active && ck == 0) {
+            store_state<P>(a, seg++, slot, r);
+            ck = a.ckpt_every;
+        }
+        const int mine = !active ? INT_MAX : (interior ? min(run, min(ck, a.n_steps - t) - 1) : 0);
+        const int extra = __reduce_min_sync(0xffffffffu, mine);
+        if (active) {
+            if (interior) {
+#pragma unroll 1
+                for (int e = 0; e <= extra; ++e) model_step<true>(a, r, cc);
+                run -= extra;
+                ck -= extra + 1;
+                t += extra + 1;
+            } else {
+                model_step<false>(a, r, cc);
+                --ck;
+                ++t;
+            }
+            if (t >= a.n_steps) active = false;
+        }
+    }
+    if (slot < a.n) {
         store_state<P>(a, a.n_seg, slot, r);
         a.nsteps[slot] = t;
-        double tt, p[3], w[3];
-        has = detector_point<P>(a, r, pa, pb, tt, p, w);
     }
-    splat_block<P>(a, has, pa, pb);
-    block_add((unsigned long long)t, &s_steps, a.total_steps);
+    warp_add((unsigned long long)t, a.total_steps);
 }
 
 // In-cell coordinates of stage 1 and the first two of stage 2 of step j of
@@ -917,28 +1064,28 @@ __global__ void __launch_bounds__(kAdjThreads, adj_fwd_min_blocks<P>()) image_fo
 // thread's column).
 template <class P>
 __device__ __forceinline__ void put_step(typename P::R* buf, int j, const StageRec<P> (&rec)[3]) {
-    typename P::R* b = buf + (size_t)j * kAdjStateWords * kAdjBwdThreads;
+    typename P::R* b = buf + (size_t)j * kAdjStateWords * kAdjThreads;
 #pragma unroll
-    for (int x = 0; x < 3; ++x) b[x * kAdjBwdThreads] = rec[0].f[x];
-    b[3 * kAdjBwdThreads] = rec[1].f[0];
-    b[4 * kAdjBwdThreads] = rec[1].f[1];
+    for (int x = 0; x < 3; ++x) b[x * kAdjThreads] = rec[0].f[x];
+    b[3 * kAdjThreads] = rec[1].f[0];
+    b[4 * kAdjThreads] = rec[1].f[1];
 }
 
 template <class P>
 __device__ __forceinline__ void get_step(const typename P::R* buf, int j, StageRec<P> (&rec)[3]) {
-    const typename P::R* b = buf + (size_t)j * kAdjStateWords * kAdjBwdThreads;
+    const typename P::R* b = buf + (size_t)j * kAdjStateWords * kAdjThreads;
 #pragma unroll
-    for (int x = 0; x < 3; ++x) rec[0].f[x] = b[x * kAdjBwdThreads];
-    rec[1].f[0] = b[3 * kAdjBwdThreads];
-    rec[1].f[1] = b[4 * kAdjBwdThreads];
+    for (int x = 0; x < 3; ++x) rec[0].f[x] = b[x * kAdjThreads];
+    rec[1].f[0] = b[3 * kAdjThreads];
+    rec[1].f[1] = b[4 * kAdjThreads];
 }
 
 template <class P, int MINB>
-__global__ void __launch_bounds__(kAdjBwdThreads, MINB) image_backward_kernel(const __grid_constant__ ImageArgs a) {
+__global__ void __launch_bounds__(kAdjThreads, MINB) image_backward_kernel(const __grid_constant__ ImageArgs a) {
     using R = typename P::R;
     extern __shared__ __align__(16) unsigned char s_dyn[];
     R* s_seg = reinterpret_cast<R*>(s_dyn) + threadIdx.x;   // this thread's column of the segment buffer
-    const long long slot = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long slot = (long long)blockIdx.x * kAdjThreads + threadIdx.x;
     if (slot >= a.n) return;
     MState<P> r;
     load_state<P>(a, a.n_seg, slot, r);
@@ -976,14 +1123,15 @@ __global__ void __launch_bounds__(kAdjBwdThreads, MINB) image_backward_kernel(co
     R segF[kMaxCkptEvery][4];
     for (int s = (T + a.ckpt_every - 1) / a.ckpt_every - 1; s >= 0; --s) {
         load_state<P>(a, s, slot, r);
-        const int j0 = s * a.ckpt_every;
-        const int m = min(a.ckpt_every, T - j0);
+        const int m = min(a.ckpt_every, T - s * a.ckpt_every);
         // recompute the segment from its checkpoint (bitwise the forward's
-        // steps), recording where each stage sampled, then run its adjoint
-        // in reverse
+        // steps), recording where each stage sampled. (A second loop without the
+        // grid tests for segments proven interior took 1e6 rays, 128^3 from 10.3 to 10.2 ms
+        // and 3e4 rays, 61^3 from 290 to 435 us: warps whose rays disagree run both.)
+        StageRec<P> rec[3];
+#pragma unroll 1
         for (int j = 0; j < m; ++j) {
-            StageRec<P> rec[3];
-            model_step<P>(a, r, cc, rec);
+            model_step<false>(a, r, cc, rec);
             put_step<P>(s_seg, j, rec);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -992,8 +1140,8 @@ __global__ void __launch_bounds__(kAdjBwdThreads, MINB) image_backward_kernel(co
             }
             segF[j][3] = rec[1].f[2];
         }
-        // segB / segF live in local memory, mostly in L2: step j - 1's
-        // records are loaded while step j's adjoint runs
+        // then its adjoint in reverse. segB / segF live in local memory, mostly
+        // in L2: step j - 1's records are loaded while step j's adjoint runs
         unsigned Bn[3];
         R Fn[4];
 #pragma unroll
@@ -1001,7 +1149,6 @@ __global__ void __launch_bounds__(kAdjBwdThreads, MINB) image_backward_kernel(co
 #pragma unroll
         for (int k = 0; k < 4; ++k) Fn[k] = segF[m - 1][k];
         for (int j = m - 1; j >= 0; --j) {
-            StageRec<P> rec[3];
             get_step<P>(s_seg, j, rec);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -1116,6 +1263,9 @@ static void fill_image_args(ImageArgs& a, const SlothGridDesc* g, const void* gr
         a.w_of_v[k] = (p->dtau / h) / kC;
         a.S[k] = -0.5 * (p->dtau / h) * (p->dtau / h);
         a.Sf[k] = (float)a.S[k];
+        a.S4f[k] = 0.25f * a.Sf[k];
+        a.S2f[k] = 0.5f * a.Sf[k];
+        a.S6f[k] = (1.0f / 6.0f) * a.Sf[k];
     }
     a.n_steps = p->n_steps;
     a.ckpt_every = p->ckpt_every;
@@ -1214,6 +1364,8 @@ static int image_forward_impl(const SlothGridDesc* g, const void* grid, const Sl
     a.accel_bound = w.bound;
     image_forward_kernel<P><<<(unsigned)((n + kAdjThreads - 1) / kAdjThreads), kAdjThreads, 0, s>>>(a);
     note_launch();
+    splat_kernel<P><<<(unsigned)((n + kSplatThreads - 1) / kSplatThreads), kSplatThreads, 0, s>>>(a);
+    note_launch();
     return cuda_status(cudaGetLastError());
 }
 
@@ -1238,11 +1390,11 @@ static int image_backward_impl(const SlothGridDesc* g, const void* grid, const S
     fill_image_args(a, g, grid, p, nullptr, n, w.perm, w.ckpt, w.nsteps);
     a.image = const_cast<typename P::R*>(image_grad);
     a.ggrad = grid_grad;
-    const size_t smem = (size_t)p->ckpt_every * kAdjStateWords * sizeof(typename P::R) * kAdjBwdThreads;
-    const unsigned blocks = (unsigned)((n + kAdjBwdThreads - 1) / kAdjBwdThreads);
+    const size_t smem = (size_t)p->ckpt_every * kAdjStateWords * sizeof(typename P::R) * kAdjThreads;
+    const unsigned blocks = (unsigned)((n + kAdjThreads - 1) / kAdjThreads);
     auto launch = [&](auto kernel) {
         cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (err == cudaSuccess) kernel<<<blocks, kAdjBwdThreads, smem, s>>>(a);
+        if (err == cudaSuccess) kernel<<<blocks, kAdjThreads, smem, s>>>(a);
         return err;
     };
     if constexpr (sizeof(typename P::R) == 4) {
@@ -1251,12 +1403,12 @@ static int image_backward_impl(const SlothGridDesc* g, const void* grid, const S
             (e = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess ||
             (e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess)
             return cuda_status(e);
-        if (4 * (smem + (size_t)reserved) <= (size_t)per_sm)
-            e = launch(image_backward_kernel<P, 4>);
+        if (16 * (smem + (size_t)reserved) <= (size_t)per_sm)
+            e = launch(image_backward_kernel<P, 16>);
         else
-            e = launch(image_backward_kernel<P, 3>);
+            e = launch(image_backward_kernel<P, 12>);
     } else {
-        e = launch(image_backward_kernel<P, 1>);
+        e = launch(image_backward_kernel<P, 8>);
     }
     if (e != cudaSuccess) return cuda_status(e);
     note_launch();

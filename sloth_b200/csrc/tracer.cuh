@@ -1199,21 +1199,6 @@ __device__ __forceinline__ void warp_add(unsigned long long v, unsigned long lon
     if ((threadIdx.x & 31) == 0 && v && dst) atomicAdd(dst, v);
 }
 
-// Sum of `v` over the block, added to *dst by one thread.
-__device__ __forceinline__ void block_add(unsigned long long v, unsigned long long* s_acc,
-                                          unsigned long long* dst) {
-    const unsigned FULL = 0xffffffffu;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
-    if ((threadIdx.x & 31) == 0 && v) atomicAdd(s_acc, v);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (dst && *s_acc) atomicAdd(dst, *s_acc);
-        *s_acc = 0;
-    }
-    __syncthreads();
-}
-
 // ---------------------------------------------------------------------------
 // Morton bucket pre-pass.
 // ---------------------------------------------------------------------------
