@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kThreads, SLOTH_TRACE_MIN_BLOCKS)
 serve_kernel(const TraceArgs* __restrict__ table, WorkHeader* hdr, const WorkItem* __restrict__ items, int mode) {
     __shared__ TraceArgs s_args;
     CellCacheFor<PolF32> cc;
-    cc.base = 0xffffffffu;
+    reset_cache(cc);
     int slot = -1;
     const int shares = hdr->count[mode] * kTileShares;
     const int offset = hdr->offset[mode];
@@ -89,7 +89,7 @@ serve_kernel(const TraceArgs* __restrict__ table, WorkHeader* hdr, const WorkIte
             const unsigned* src = reinterpret_cast<const unsigned*>(table + slot);
             unsigned* dst = reinterpret_cast<unsigned*>(&s_args);
             for (int i = threadIdx.x; i < (int)(sizeof(TraceArgs) / 4); i += 32) dst[i] = src[i];
-            cc.base = 0xffffffffu;
+            reset_cache(cc);
             __syncwarp();
         }
         const unsigned start = (unsigned)it.tile * kTile + (unsigned)(w % kTileShares) * kWarpRays;

@@ -4,21 +4,36 @@
 
 namespace sloth {
 
-template <class P, int IB, int FAST, int INTEG>
-__global__ void __launch_bounds__(kThreads, trace_min_blocks<P, INTEG>())
+// Which FP32 build traces n rays with Runge-Kutta-Nystrom steps: the one that
+// fetches the next cell ahead while its 12 warps per SM hold all the rays at once,
+// the 16-warp one above. With few warps a step waits for its cell (long scoreboard
+// a third of it); with 16 the load and store pipe has no room for the ring's
+// extra copies. Measured without / with: 3e3 rays, 128^3 127 / 103 us; 1e4 129 / 105;
+// 192^3 turbulent, 3e4 526 / 470, 5.6e4 575 / 523, 7.2e4 627 / 682; along x, 2e4 rays
+// 679 / 536 us; 512^3, 1e7 rays 105 / 119 ms.
+constexpr int kAheadWarps = 12;
+// Rays of a warp's first take: 32, or as few as kSpreadMin as long as that gives
+// each of an SM's four schedulers one warp (fewer rays, fewer cells that the warp waits
+// for: FP64, 5e3 rays 597 -> 529 us; 1e4 rays, 128^3 107 -> 105). More, smaller warps
+// share the schedulers and lose: 1e4 rays in warps of 8 (two per scheduler) 133 us.
+constexpr int kSpreadWarps = 4, kSpreadMin = 8;
+
+template <class P, int IB, int FAST, int INTEG, bool AHEAD>
+__global__ void __launch_bounds__(kThreads, trace_min_blocks<P, INTEG, AHEAD>())
 trace_kernel(const __grid_constant__ TraceArgs a, int first_rays) {
     unsigned long long my_steps = 0;
-    CellCacheFor<P> cc;
-    cc.base = 0xffffffffu;
+    CellCacheFor<P, AHEAD> cc;
+    reset_cache(cc);
     const unsigned n = (unsigned)a.n;
     const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const unsigned warps = gridDim.x * (kThreads / 32);
     TraceQueue q{a.queue, warps * first_rays, min(warp * first_rays, n), min((warp + 1) * first_rays, n), n};
     trace_warp<P, IB, FAST, INTEG>(a, q, cc, my_steps);
+    if constexpr (AHEAD) fetch_wait();
     warp_add(my_steps, a.total_steps);
 }
 
-template <class P, int IB, int FAST, int INTEG>
+template <class P, int IB, int FAST, int INTEG, bool AHEAD>
 static int launch_trace_k(const TraceArgs& ta, int sms, cudaStream_t s) {
     static int cached[64] = {0};
     int dev = 0;
@@ -26,31 +41,35 @@ static int launch_trace_k(const TraceArgs& ta, int sms, cudaStream_t s) {
     if (e != cudaSuccess) return cuda_status(e);
     int per_sm = (dev >= 0 && dev < 64) ? cached[dev] : 0;
     if (per_sm <= 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<P, IB, FAST, INTEG>, kThreads, 0) !=
-                cudaSuccess || per_sm < 1)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<P, IB, FAST, INTEG, AHEAD>, kThreads,
+                                                          0) != cudaSuccess || per_sm < 1)
             per_sm = 1;
         if (dev >= 0 && dev < 64) cached[dev] = per_sm;
     }
     long long blocks = (long long)sms * per_sm;
-    const int first = 32;
-    const long long want = (ta.n + first * (kThreads / 32) - 1) / (first * (kThreads / 32));
+    int first = 32;
+    const long long spread = (ta.n + (long long)sms * kSpreadWarps - 1) / ((long long)sms * kSpreadWarps);
+    if (spread < first) first = spread > kSpreadMin ? (int)spread : kSpreadMin;
+    const long long want = (ta.n + first - 1) / first;
     if (blocks > want) blocks = want;
-    trace_kernel<P, IB, FAST, INTEG><<<(int)blocks, kThreads, 0, s>>>(ta, first);
+    trace_kernel<P, IB, FAST, INTEG, AHEAD><<<(int)blocks, kThreads, 0, s>>>(ta, first);
     note_launch();
     return cuda_status(cudaGetLastError());
 }
 
-template <class P, int IB, int INTEG>
+template <class P, int IB, int INTEG, bool AHEAD = false>
 static int launch_trace_i(const TraceArgs& ta, int sms, cudaStream_t s, int fast) {
-    return fast == 1 ? launch_trace_k<P, IB, 1, INTEG>(ta, sms, s)
-         : fast == 2 ? launch_trace_k<P, IB, 2, INTEG>(ta, sms, s)
-                     : launch_trace_k<P, IB, 0, INTEG>(ta, sms, s);
+    return fast == 1 ? launch_trace_k<P, IB, 1, INTEG, AHEAD>(ta, sms, s)
+         : fast == 2 ? launch_trace_k<P, IB, 2, INTEG, AHEAD>(ta, sms, s)
+                     : launch_trace_k<P, IB, 0, INTEG, AHEAD>(ta, sms, s);
 }
 
 template <class P, int IB>
 static int launch_trace(const TraceArgs& ta, int sms, cudaStream_t s, int fast, int integ) {
-    return integ == INTEG_RK4 ? launch_trace_i<P, IB, INTEG_RK4>(ta, sms, s, fast)
-                              : launch_trace_i<P, IB, INTEG_RKN>(ta, sms, s, fast);
+    if (integ == INTEG_RK4) return launch_trace_i<P, IB, INTEG_RK4>(ta, sms, s, fast);
+    if constexpr (sizeof(typename P::R) == 4)
+        if (ta.n <= (long long)sms * kAheadWarps * 32) return launch_trace_i<P, IB, INTEG_RKN, true>(ta, sms, s, fast);
+    return launch_trace_i<P, IB, INTEG_RKN>(ta, sms, s, fast);
 }
 
 template <class P>

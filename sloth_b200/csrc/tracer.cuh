@@ -88,6 +88,8 @@ struct TraceArgs {
     long long n;
     const unsigned* perm;      // bucket-ordered ray ids
     unsigned* queue;           // rays handed out beyond each warp's first ones
+    unsigned sa, s1, s2;       // voxel strides along the probing axis and the transverse axes t1, t2
+    unsigned ahead_max;        // last voxel at which a fetched face may start
     double origin[3], spacing[3];
     double w_of_v[3];          // w = v * w_of_v   (cells per step per m/s)
     double v_of_w[3];          // v = w * v_of_w
@@ -209,6 +211,13 @@ struct CellPolyF2 {
     float2 t[2][8];
 };
 
+// The same with the next cell along the probing axis fetched ahead (see
+// cell_fill).
+struct CellAheadF2 : CellPolyF2 {
+    unsigned pred;      // the cell whose far face is on its way
+    unsigned slot;      // byte offset of the cell's near face in s_face
+};
+
 // The cell's kappa polynomial stays in shared memory rather than registers:
 // each thread owns one slot, [2][threads] float4 (FP64: [4][threads] double2) so
 // that a warp's 16-byte loads do not conflict. This keeps 8 values out of the
@@ -300,17 +309,11 @@ __device__ __forceinline__ R corner_x2(R n1) {
     if constexpr (sizeof(R) == 4) return __fmul_rn(x, x); else return __dmul_rn(x, x);
 }
 
-// Loads cell b into the paired cache: its polynomial coefficients, two
-// channels per instruction.
-template <class P, int IB>
-__device__ __forceinline__ void paired_fill(const TraceArgs& a, unsigned b, CellPolyF2& cc) {
-    const GridGeo& g = a.geo;
-    cc.base = b;
-    const float4* gp = reinterpret_cast<const float4*>(a.grid);
-    const float4 v0 = __ldg(gp + b), v1 = __ldg(gp + b + 1u);
-    const float4 v2 = __ldg(gp + b + g.sy), v3 = __ldg(gp + b + g.sy + 1u);
-    const float4 v4 = __ldg(gp + b + g.sx), v5 = __ldg(gp + b + g.sx + 1u);
-    const float4 v6 = __ldg(gp + b + g.sx + g.sy), v7 = __ldg(gp + b + g.sx + g.sy + 1u);
+// The paired cache's polynomials from a cell's corners (index 4*dx + 2*dy + dz),
+// two channels per instruction.
+template <int IB>
+__device__ __forceinline__ void paired_coeffs(const TraceArgs& a, CellPolyF2& cc, float4 v0, float4 v1, float4 v2,
+                                              float4 v3, float4 v4, float4 v5, float4 v6, float4 v7) {
 #define SLOTH_LO(v) make_float2(v.x, v.y)
 #define SLOTH_HI(v) make_float2(v.z, v.w)
     poly_coeffs2(cc.t[0], SLOTH_LO(v0), SLOTH_LO(v1), SLOTH_LO(v2), SLOTH_LO(v3), SLOTH_LO(v4), SLOTH_LO(v5),
@@ -326,11 +329,93 @@ __device__ __forceinline__ void paired_fill(const TraceArgs& a, unsigned b, Cell
         kappa_store(k);
     } else if constexpr (IB == IB_GENERAL) {
         float k[8];
-        poly_coeffs<float>(k, corner_kappa<P>(a, v0.x), corner_kappa<P>(a, v1.x), corner_kappa<P>(a, v2.x),
-                           corner_kappa<P>(a, v3.x), corner_kappa<P>(a, v4.x), corner_kappa<P>(a, v5.x),
-                           corner_kappa<P>(a, v6.x), corner_kappa<P>(a, v7.x));
+        poly_coeffs<float>(k, corner_kappa<PolF32>(a, v0.x), corner_kappa<PolF32>(a, v1.x), corner_kappa<PolF32>(a, v2.x),
+                           corner_kappa<PolF32>(a, v3.x), corner_kappa<PolF32>(a, v4.x), corner_kappa<PolF32>(a, v5.x),
+                           corner_kappa<PolF32>(a, v6.x), corner_kappa<PolF32>(a, v7.x));
         kappa_store(k);
     }
+}
+
+// A corner of the packed grid. The 256-byte hint has L2 fetch the neighbouring
+// 128 bytes (eight voxels further along z) from memory with a missing line: 512^3 / 1e7
+// rays 105.0 -> 104.0 ms, 3e5 rays 4.53 -> 4.38 ms, 192^3 / 8e4 755 -> 741 us.
+__device__ __forceinline__ float4 load_corner(const float4* p) {
+    float4 v;
+    asm("ld.global.nc.L2::256B.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+// Loads cell b into the paired cache.
+template <int IB>
+__device__ __forceinline__ void cell_fill(const TraceArgs& a, unsigned b, CellPolyF2& cc) {
+    const GridGeo& g = a.geo;
+    const float4* gp = reinterpret_cast<const float4*>(a.grid) + b;
+    cc.base = b;
+    paired_coeffs<IB>(a, cc, load_corner(gp), load_corner(gp + 1u), load_corner(gp + g.sy), load_corner(gp + g.sy + 1u),
+                      load_corner(gp + g.sx), load_corner(gp + g.sx + 1u), load_corner(gp + g.sx + g.sy),
+                      load_corner(gp + g.sx + g.sy + 1u));
+}
+
+// Faces of cells across the probing axis in shared memory: a ring of three per
+// thread, four corners each, [face][corner][lane] so that a warp's 16-byte accesses do not
+// conflict. Corner 2*d1 + d2 sits d1, d2 points along the transverse axes.
+constexpr unsigned kFaceRow = 32u * 16u, kFaceBytes = 4u * kFaceRow;
+static __shared__ float4 s_face[3][4][32];
+
+__device__ __forceinline__ unsigned face_after(unsigned f) { return f == 2u * kFaceBytes ? 0u : f + kFaceBytes; }
+
+__device__ __forceinline__ void fetch_face(unsigned to, const float4* from, const TraceArgs& a) {
+    auto copy = [](unsigned d, const float4* p) {
+        asm volatile("cp.async.ca.shared.global.L2::256B [%0], [%1], 16;" ::"r"(d), "l"(p) : "memory");
+    };
+    copy(to, from);
+    copy(to + kFaceRow, from + a.s2);
+    copy(to + 2u * kFaceRow, from + a.s1);
+    copy(to + 3u * kFaceRow, from + a.s1 + a.s2);
+}
+
+__device__ __forceinline__ float4 face_corner(unsigned at) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+
+// Waits for this thread's copies; the last prefetched face may still be on its
+// way when its warp runs out of rays.
+__device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The fill of kernels whose warps wait for memory rather than for issue slots:
+// a ray mostly moves on to the next cell along the probing axis, whose near face is
+// this cell's far face, so each fill asks for the far face after that one and
+// finds its own, asked for about two steps earlier, in shared memory. Any other
+// cell's two faces are fetched now. The same corners, so bitwise the same rays.
+template <int IB>
+__device__ __forceinline__ void cell_fill(const TraceArgs& a, unsigned b, CellAheadF2& cc) {
+    const float4* gp = reinterpret_cast<const float4*>(a.grid);
+    const unsigned own = (unsigned)__cvta_generic_to_shared(&s_face[0][0][threadIdx.x & 31]);
+    unsigned near = cc.slot;
+    if (b == cc.pred) {
+        near = face_after(near);
+    } else {
+        fetch_face(own + near, gp + b, a);
+        fetch_face(own + face_after(near), gp + b + a.sa, a);
+    }
+    const unsigned far = face_after(near);
+    fetch_wait();
+    const unsigned along = far - near;       // modulo 2^32
+    const unsigned dx = a.axis == 0 ? along : 2u * kFaceRow;
+    const unsigned dy = a.axis == 1 ? along : (a.axis == 0 ? 2u * kFaceRow : kFaceRow);
+    const unsigned dz = a.axis == 2 ? along : kFaceRow;
+    const unsigned at = own + near;
+    const float4 v0 = face_corner(at), v1 = face_corner(at + dz), v2 = face_corner(at + dy), v3 = face_corner(at + dy + dz);
+    const float4 v4 = face_corner(at + dx), v5 = face_corner(at + dx + dz), v6 = face_corner(at + dx + dy),
+                 v7 = face_corner(at + dx + dy + dz);
+    // clamped into the grid: beyond it there is no cell that would use the face
+    fetch_face(own + face_after(far), gp + min(b + 2u * a.sa, a.ahead_max), a);
+    cc.base = b;
+    cc.pred = b + a.sa;
+    cc.slot = near;
+    paired_coeffs<IB>(a, cc, v0, v1, v2, v3, v4, v5, v6, v7);
 }
 
 // FP64 trilinear sample of the packed grid (rules of src/core/interpolator.py:79-104:
@@ -498,9 +583,9 @@ __device__ __forceinline__ void rkn_step(const TraceArgs& a, Ray<P>& r, Cache& c
 __device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
 
 // sample at (hx + lx, hyz + lyz)
-template <int IB, int MODE>
+template <int IB, int MODE, class Cache>
 __device__ __forceinline__ void sample_f2(const TraceArgs& a, float hx, float lx, float2 hyz, float2 lyz,
-                                          Sample<PolF32>& out, CellPolyF2& cc) {
+                                          Sample<PolF32>& out, Cache& cc) {
     const GridGeo& g = a.geo;
     float px = hx + lx;
     float2 pyz = __fadd2_rn(hyz, lyz);
@@ -531,7 +616,7 @@ __device__ __forceinline__ void sample_f2(const TraceArgs& a, float hx, float lx
     const float fx = (hx - (float)ix) + lx;
     const float2 fyz = __fadd2_rn(__fadd2_rn(hyz, make_float2(-(float)iy, -(float)iz)), lyz);
     const unsigned b = (unsigned)ix * g.sx + (unsigned)iy * g.sy + (unsigned)iz;
-    if (b != cc.base) paired_fill<PolF32, IB>(a, b, cc);
+    if (b != cc.base) cell_fill<IB>(a, b, cc);
     const float2 fx2 = bc2(fx), fy2 = bc2(fyz.x), fz2 = bc2(fyz.y);
     const float2 r0 = poly_eval2(cc.t[0], fx2, fy2, fz2);
     const float2 r1 = poly_eval2(cc.t[1], fx2, fy2, fz2);
@@ -567,8 +652,8 @@ __device__ __forceinline__ void kahan2_fma(float2& s, float2& c, float2 a, float
 // UNIT: phi is 1 (every step but a cut one); the multiplications by phi are
 // left out, which gives bitwise the results of the general form at phi = 1
 // (fma(1, a, b) rounds as a + b).
-template <int IB, int MODE, bool UNIT>
-__device__ __forceinline__ void rkn_step_f2(const TraceArgs& a, Ray<PolF32>& r, CellPolyF2& cc, float phi) {
+template <int IB, int MODE, bool UNIT, class Cache>
+__device__ __forceinline__ void rkn_step_f2(const TraceArgs& a, Ray<PolF32>& r, Cache& cc, float phi) {
     if constexpr (UNIT) phi = 1.0f;
     auto mphi = [&](float x) { return UNIT ? x : __fmul_rn(phi, x); };
     auto mphi2 = [&](float2 x) { return UNIT ? x : __fmul2_rn(bc2(phi), x); };
@@ -740,8 +825,8 @@ __device__ __forceinline__ void rk4_step(const TraceArgs& a, Ray<P>& r, Cache& c
 
 // The RK4 step in the paired FP32 form (y and z components as register
 // pairs), every rounding explicit.
-template <int IB, int MODE, bool UNIT>
-__device__ __forceinline__ void rk4_step_f2(const TraceArgs& a, Ray<PolF32>& r, CellPolyF2& cc, float phi) {
+template <int IB, int MODE, bool UNIT, class Cache>
+__device__ __forceinline__ void rk4_step_f2(const TraceArgs& a, Ray<PolF32>& r, Cache& cc, float phi) {
     if constexpr (UNIT) phi = 1.0f;
     auto mphi = [&](float x) { return UNIT ? x : __fmul_rn(phi, x); };
     auto mphi2 = [&](float2 x) { return UNIT ? x : __fmul2_rn(bc2(phi), x); };
@@ -1181,15 +1266,24 @@ __device__ __forceinline__ void trace_warp(const TraceArgs& a, Queue& q, Cache& 
     }
 }
 
-// The cell cache of a precision.
-template <class P>
-using CellCacheFor = typename std::conditional<sizeof(typename P::R) == 4, CellPolyF2, CellPolyD>::type;
+// The cell cache of a precision; AHEAD: FP32 with the next cell fetched ahead.
+template <class P, bool AHEAD = false>
+using CellCacheFor = typename std::conditional<sizeof(typename P::R) != 4, CellPolyD,
+                                               typename std::conditional<AHEAD, CellAheadF2, CellPolyF2>::type>::type;
 
-// One-warp CTAs per SM: FP32 at 128 registers; FP64 at 168, which holds the
+__device__ __forceinline__ void reset_cache(CellPolyD& cc) { cc.base = 0xffffffffu; }
+__device__ __forceinline__ void reset_cache(CellPolyF2& cc) { cc.base = 0xffffffffu; }
+__device__ __forceinline__ void reset_cache(CellAheadF2& cc) {
+    cc.base = cc.pred = 0xffffffffu;
+    cc.slot = 0u;
+}
+
+// One-warp CTAs per SM: FP32 at 128 registers (152 with the next cell fetched
+// ahead); FP64 at 168, which holds the
 // polynomials without spilling (256^3 / 4e5 rays: 4.53 ms, against 5.33 ms
 // at 128 registers and 16 warps with 330 B of spill, 4.61 at 10 warps, 4.98 at 8).
-template <class P, int INTEG> constexpr int trace_min_blocks() {
-    return sizeof(typename P::R) == 4 ? SLOTH_TRACE_MIN_BLOCKS : (INTEG == INTEG_RK4 ? 8 : 12);
+template <class P, int INTEG, bool AHEAD> constexpr int trace_min_blocks() {
+    return sizeof(typename P::R) == 4 ? (AHEAD ? 12 : SLOTH_TRACE_MIN_BLOCKS) : (INTEG == INTEG_RK4 ? 8 : 12);
 }
 
 // Sum of `v` over the warp, added to *dst by one lane.
@@ -1414,6 +1508,11 @@ inline void fill_trace_args(TraceArgs& ta, const SlothGridDesc* g, const void* g
     ta.n = n;
     ta.perm = perm;
     ta.queue = nullptr;
+    const unsigned stride[3] = {ta.geo.sx, ta.geo.sy, 1u};
+    ta.sa = stride[axis];
+    ta.s1 = stride[axis == 0 ? 1 : 0];
+    ta.s2 = stride[axis == 2 ? 1 : 2];
+    ta.ahead_max = (unsigned)g->n[0] * (unsigned)g->n[1] * (unsigned)g->n[2] - 1u - ta.s1 - ta.s2;
     for (int k = 0; k < 3; ++k) {
         const double h = g->spacing[k];
         ta.origin[k] = g->origin[k];

@@ -1,7 +1,8 @@
-"""The tracer's ray queue and pre-pass at the sizes where they change: part
-of a warp, one ray around whole warps and around the rays that a full GPU's
-warps take first, and around the pre-pass's bucket counts (a scan of one word,
-of one and of several CTAs). Each ray's result does not depend on the other rays of its
+"""The tracer's ray queue, pre-pass and builds at the sizes where they change: part
+of a warp, one ray around whole warps, around the rays that a full GPU's warps take
+first, around the largest trace of the build that fetches the next cell ahead (with rays
+along each axis and some that run backwards), and around the pre-pass's bucket counts
+(a scan of one word, of one and of several CTAs). Each ray's result does not depend on the other rays of its
 launch, so every size gives bitwise the rays of one larger trace."""
 import pytest
 import torch
@@ -22,21 +23,30 @@ def _trace(n_rays, rays, grid, sched, **kw):
 
 
 @pytest.mark.parametrize("precision", ["f32", "f64"])
-@pytest.mark.parametrize("shape", [(20, 33, 24), (2, 2, 40)])
-def test_every_ray_once_and_bitwise_the_same(precision, shape):
+@pytest.mark.parametrize("shape,axis,ib", [((20, 33, 24), 2, True), ((2, 2, 40), 2, False), ((31, 18, 27), 0, True),
+                                           ((19, 22, 30), 1, False)])
+def test_every_ray_once_and_bitwise_the_same(precision, shape, axis, ib):
     h = tuple(L / (k - 1) for k in shape)
     g = torch.Generator().manual_seed(3)
     ne = (torch.rand(shape, generator=g) * 2e25).float()
     grid = runtime.pack_grid(ne, (-L / 2,) * 3, h, physics.omega_of(532e-9), precision=precision)
     most = 148 * 16 * 32 + 33            # a B200's warps at 16 per SM, and one more warp's worth
     rays = workloads.gaussian_beam(most, waist=3e-3, L=L, jitter=5e-2, seed=2, device="cuda", dtype=torch.float64)
+    to = {0: [2, 0, 1], 1: [0, 2, 1], 2: [0, 1, 2]}[axis]      # the beam along `axis`
+    rays = rays[to + [3 + k for k in to]].contiguous()
+    back = torch.arange(most, device="cuda") % 7 == 3           # some rays run backwards from the far face
+    rays[axis, back] = L / 2
+    rays[3 + axis, back] *= -1.0
     rays = rays.to(torch.float32 if precision == "f32" else torch.float64)
     sched = runtime.schedule_times([0.0, L, 2 * L], h)
-    whole = _trace(most, rays, grid, sched)
+    kw = dict(axis=axis, inv_brems=ib, Te=20.0 if ib else None, Z=1.0 if ib else None)
+    keys = ["jones", "phase", "status", "steps"] + (["amp"] if ib else [])
+    whole = _trace(most, rays, grid, sched, **kw)
     assert int(whole["total_steps"]) == int(whole["steps"].sum(dtype=torch.int64))
-    for n in (1, 2, 8, 9, 31, 32, 33, 64, 255, 257, 32768, 32769, 65537, 148 * 12 * 32 + 1, most - 33, most - 1):
-        part = _trace(n, rays, grid, sched)
-        for k in ("jones", "phase", "status", "steps"):
+    for n in (1, 2, 8, 9, 31, 32, 33, 64, 255, 257, 4737, 18944, 18945, 32768, 32769, 148 * 12 * 32, 148 * 12 * 32 + 1,
+              65537, most - 33, most - 1):
+        part = _trace(n, rays, grid, sched, **kw)
+        for k in keys:
             assert torch.equal(part[k], whole[k][..., :n]), (n, k)
         assert int(part["total_steps"]) == int(part["steps"].sum(dtype=torch.int64))
     assert int(whole["status"].max()) <= 2 and float(whole["jones"].abs().max()) < 1e9
