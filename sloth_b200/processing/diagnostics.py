@@ -233,7 +233,7 @@ class Diagnostic:
                 print(f" --> {round((1 - self.Np_inc / self.Np) * 100, 3)} % filtered before diagnostic solve.")
         self._rf_in = t                   # device, metres, caller's precision
         self._weights_dev = w
-        self.weights = None if w is None else w.cpu().numpy()
+        self.weights = None if w is None else runtime.download(w)
         self._ops: Optional[List[Op]] = None
         self._rf_custom = None
         self._rf_cache = None
@@ -243,7 +243,7 @@ class Diagnostic:
     def r0(self):
         if self._rf_in is None:
             return None
-        return m_to_mm(self._rf_in.cpu().numpy())
+        return m_to_mm(runtime.download(self._rf_in))
 
     @property
     def rf(self):
