@@ -82,7 +82,7 @@ def _image_forward(ne: torch.Tensor, rays: torch.Tensor, origin, spacing, omega:
     if rays.dim() != 2 or rays.shape[0] != 6:
         raise ValueError("rays must be (6, N)")
     grid = runtime.pack_grid(ne.detach(), origin, spacing, omega, precision=precision, device=ne.device,
-                             layout="values")
+                             layout="values", with_range=False)   # the forward bounds its accelerations itself
     params = spec.params()
     n = int(rays.shape[1])
     ws_bytes = int(capi.load().sloth_image_workspace_bytes(ctypes.byref(params), n))

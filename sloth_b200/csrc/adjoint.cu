@@ -705,7 +705,9 @@ __device__ __forceinline__ bool detector_point(const ImageArgs& a, const MState<
 // the other, its lanes on consecutive taps, so that a reduction covers whole rows of
 // the window.
 constexpr int kSplatRounds = 6;
-constexpr int kSplatMin = 8;                  // rays that are worth a tile
+// Rays that are worth a tile: its pixels are added once each, twice as many
+// taps or more go into it.
+__device__ __forceinline__ int splat_min(int taps) { return max(8, 2 * 32 * 32 / (taps * taps)); }
 constexpr int kSplatThreads = 256;
 constexpr int kSplatTile = 32;                // pixels per side of a block's tile
 constexpr int kSplatPitch = kSplatTile + 4;   // 16-byte rows
@@ -788,7 +790,7 @@ __global__ void __launch_bounds__(kSplatThreads) splat_kernel(const __grid_const
             s_b[at] = pb;
         }
         __syncthreads();
-        if (members < kSplatMin) {         // not worth a tile (none when the window is larger than it)
+        if (members < splat_min(a.taps)) {         // not worth a tile (none when the window is larger than it)
             direct = direct || tiled || t == lead;
             left_over = left_over && !direct;
             continue;

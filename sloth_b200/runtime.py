@@ -125,14 +125,16 @@ def _from_order_key(key: int) -> float:
 
 def pack_grid(ne, origin, spacing, omega, *, precision="f32", device=None, stream=None,
               out: Optional[torch.Tensor] = None, ne_scale: Optional[float] = None,
-              layout: str = "trace") -> DeviceGrid:
+              layout: str = "trace", with_range: bool = True) -> DeviceGrid:
     """K1: pack ne (m^-3, (nx, ny, nz) array or tensor) into a device grid.
 
     ``ne`` may be a numpy array, a CPU tensor (pinned for a fast copy) or a
     CUDA tensor; float32 and float64 are read as they are. q = ne * ne_scale
     with ne_scale = 1/nc(omega) unless given. ``layout`` 'trace' (the
     tracers' grid) stores n - 1 of the plasma refractive index in channel 0,
-    'values' stores q there (for the K0 sampler).
+    'values' stores q there (for the K0 sampler). The density's range, which
+    the tracers' fast paths use, is the one thing the call waits for;
+    ``with_range=False`` leaves it unknown and does not wait.
     """
     if layout not in ("trace", "values"):
         raise ValueError("layout must be 'trace' or 'values'")
@@ -156,18 +158,28 @@ def pack_grid(ne, origin, spacing, omega, *, precision="f32", device=None, strea
         out = torch.empty(nbytes // rb, dtype=torch.float32 if rb == 4 else torch.float64, device=dev)
     scale = 1.0 / physics.critical_density(omega) if ne_scale is None else float(ne_scale)
     lib = capi.load()
+    ope2 = physics.ope_ratio2(omega) if layout == "trace" else 0.0
+    geom = (out, desc, precision, float(omega), n, tuple(map(float, origin)), tuple(map(float, spacing)))
     run_on = stream if stream is not None else torch.cuda.current_stream(dev)
     if stream is not None:
         run_on.wait_stream(torch.cuda.current_stream(dev))   # ne and out belong to the current stream
+    if not with_range:
+        if layout == "trace":
+            fn = lib.sloth_grid_pack_trace_f32 if rb == 4 else lib.sloth_grid_pack_trace_f64
+            rc = fn(desc, capi.ptr(ne), int(ne.dtype == torch.float64), scale, ope2, capi.ptr(out), _stream_ptr(run_on))
+        else:
+            fn = lib.sloth_grid_pack_f32 if rb == 4 else lib.sloth_grid_pack_f64
+            rc = fn(desc, capi.ptr(ne), int(ne.dtype == torch.float64), scale, capi.ptr(out), _stream_ptr(run_on))
+        capi.check(rc, "sloth_grid_pack")
+        return DeviceGrid(*geom, layout=layout)
     with torch.cuda.stream(run_on):
         rng = torch.empty(2, dtype=torch.int64, device=dev)
         capi.check(lib.sloth_grid_pack_range(desc, capi.ptr(ne), int(ne.dtype == torch.float64), int(rb == 8), scale,
-                                             physics.ope_ratio2(omega) if layout == "trace" else 0.0, capi.ptr(out),
-                                             capi.ptr(rng), _stream_ptr(run_on)), "sloth_grid_pack_range")
+                                             ope2, capi.ptr(out), capi.ptr(rng), _stream_ptr(run_on)),
+                   "sloth_grid_pack_range")
         ne_max, neg_min = (_from_order_key(k) for k in rng.tolist())   # the one wait of the call
     q_max, q_min = ne_max * scale, -neg_min * scale
-    return DeviceGrid(out, desc, precision, float(omega), n, tuple(map(float, origin)), tuple(map(float, spacing)),
-                      q_max=max(q_max, 0.0) * (1.0 + 1e-6), q_min=min(q_min, 0.0) * (1.0 + 1e-6), ne_max=ne_max,
+    return DeviceGrid(*geom, q_max=max(q_max, 0.0) * (1.0 + 1e-6), q_min=min(q_min, 0.0) * (1.0 + 1e-6), ne_max=ne_max,
                       layout=layout)
 
 
