@@ -61,10 +61,9 @@ struct WorkHeader {
 constexpr int kTile = 1024;               // rays per work item
 constexpr int kWarpRays = 32;
 constexpr int kTileShares = kTile / kWarpRays;
-static_assert(kThreads == 32, "a serving CTA is one warp");
 
 template <int IB, int FAST>
-__global__ void __launch_bounds__(kThreads, SLOTH_TRACE_MIN_BLOCKS)
+__global__ void __launch_bounds__(32, kWarpsPerSm)
 serve_kernel(const TraceArgs* __restrict__ table, WorkHeader* hdr, const WorkItem* __restrict__ items, int mode) {
     __shared__ TraceArgs s_args;
     CellCacheFor<PolF32> cc;
@@ -286,12 +285,12 @@ static int graph_build(ServerImpl* s, IterSlot& is, int blocks[kModes]) {
         for (int m = 0; m < kModes; ++m) {
             cudaStreamWaitEvent(side[m], fork, 0);
             switch (m) {
-                case 2 * IB_OFF: serve_kernel<IB_OFF, 0><<<blocks[m], kThreads, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
-                case 2 * IB_OFF + 1: serve_kernel<IB_OFF, 1><<<blocks[m], kThreads, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
-                case 2 * IB_SUBCRITICAL: serve_kernel<IB_SUBCRITICAL, 0><<<blocks[m], kThreads, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
-                case 2 * IB_SUBCRITICAL + 1: serve_kernel<IB_SUBCRITICAL, 1><<<blocks[m], kThreads, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
-                case 2 * IB_GENERAL: serve_kernel<IB_GENERAL, 0><<<blocks[m], kThreads, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
-                default: serve_kernel<IB_GENERAL, 1><<<blocks[m], kThreads, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
+                case 2 * IB_OFF: serve_kernel<IB_OFF, 0><<<blocks[m], 32, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
+                case 2 * IB_OFF + 1: serve_kernel<IB_OFF, 1><<<blocks[m], 32, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
+                case 2 * IB_SUBCRITICAL: serve_kernel<IB_SUBCRITICAL, 0><<<blocks[m], 32, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
+                case 2 * IB_SUBCRITICAL + 1: serve_kernel<IB_SUBCRITICAL, 1><<<blocks[m], 32, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
+                case 2 * IB_GENERAL: serve_kernel<IB_GENERAL, 0><<<blocks[m], 32, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
+                default: serve_kernel<IB_GENERAL, 1><<<blocks[m], 32, 0, side[m]>>>(s->d_table, is.d_buf, items, m); break;
             }
             cudaEventRecord(join[m], side[m]);
             cudaStreamWaitEvent(is.stream, join[m], 0);
@@ -311,7 +310,7 @@ static int graph_build(ServerImpl* s, IterSlot& is, int blocks[kModes]) {
 template <int IB, int FAST>
 static int resident_blocks(int sms) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, serve_kernel<IB, FAST>, kThreads, 0) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, serve_kernel<IB, FAST>, 32, 0) != cudaSuccess ||
         b < 1)
         b = 1;
     return b * sms;

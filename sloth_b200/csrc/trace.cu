@@ -19,14 +19,14 @@ constexpr int kAheadWarps = 12;
 constexpr int kSpreadWarps = 4, kSpreadMin = 8;
 
 template <class P, int IB, int FAST, int INTEG, bool AHEAD>
-__global__ void __launch_bounds__(kThreads, trace_min_blocks<P, INTEG, AHEAD>())
+__global__ void __launch_bounds__(trace_threads<P, AHEAD>(), trace_min_blocks<P, INTEG, AHEAD>())
 trace_kernel(const __grid_constant__ TraceArgs a, int first_rays) {
     unsigned long long my_steps = 0;
     CellCacheFor<P, AHEAD> cc;
     reset_cache(cc);
     const unsigned n = (unsigned)a.n;
-    const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    const unsigned warps = gridDim.x * (kThreads / 32);
+    constexpr unsigned kWarps = trace_threads<P, AHEAD>() / 32;
+    const unsigned warp = blockIdx.x * kWarps + (threadIdx.x >> 5), warps = gridDim.x * kWarps;
     TraceQueue q{a.queue, warps * first_rays, min(warp * first_rays, n), min((warp + 1) * first_rays, n), n};
     trace_warp<P, IB, FAST, INTEG>(a, q, cc, my_steps);
     if constexpr (AHEAD) fetch_wait();
@@ -35,14 +35,14 @@ trace_kernel(const __grid_constant__ TraceArgs a, int first_rays) {
 
 template <class P, int IB, int FAST, int INTEG, bool AHEAD>
 static int launch_trace_k(const TraceArgs& ta, int sms, cudaStream_t s) {
+    constexpr int kCta = trace_threads<P, AHEAD>(), kWarps = kCta / 32;
     static int cached[64] = {0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_status(e);
     int per_sm = (dev >= 0 && dev < 64) ? cached[dev] : 0;
     if (per_sm <= 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<P, IB, FAST, INTEG, AHEAD>, kThreads,
-                                                          0) != cudaSuccess || per_sm < 1)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_kernel<P, IB, FAST, INTEG, AHEAD>, kCta, 0) != cudaSuccess || per_sm < 1)
             per_sm = 1;
         if (dev >= 0 && dev < 64) cached[dev] = per_sm;
     }
@@ -50,9 +50,9 @@ static int launch_trace_k(const TraceArgs& ta, int sms, cudaStream_t s) {
     int first = 32;
     const long long spread = (ta.n + (long long)sms * kSpreadWarps - 1) / ((long long)sms * kSpreadWarps);
     if (spread < first) first = spread > kSpreadMin ? (int)spread : kSpreadMin;
-    const long long want = (ta.n + first - 1) / first;
+    const long long want = (ta.n + first * kWarps - 1) / (first * kWarps);
     if (blocks > want) blocks = want;
-    trace_kernel<P, IB, FAST, INTEG, AHEAD><<<(int)blocks, kThreads, 0, s>>>(ta, first);
+    trace_kernel<P, IB, FAST, INTEG, AHEAD><<<(int)blocks, kCta, 0, s>>>(ta, first);
     note_launch();
     return cuda_status(cudaGetLastError());
 }

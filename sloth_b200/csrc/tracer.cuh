@@ -28,7 +28,7 @@
 //   1. keys_kernel   : Morton key of each ray's entry cell + bucket histogram
 //   2. scan_kernel   : exclusive scan of the bucket counts
 //   3. scatter_kernel: ray ids into bucket order
-//   4. trace_kernel  : persistent one-warp CTAs; each warp traces 32
+//   4. trace_kernel  : persistent CTAs of one or two warps; each warp traces 32
 //                      neighbouring rays of the bucket order, one thread per
 //                      ray, and refills finished lanes from the queue with one
 //                      warp ballot + one atomic (see trace_warp).
@@ -51,8 +51,9 @@
 #endif
 namespace sloth {
 
-constexpr int kThreads = SLOTH_TRACE_THREADS;   // one warp per CTA
-constexpr int kRefill = SLOTH_REFILL;            // idle lanes that a warp refills together
+constexpr int kThreads = 64;     // threads of the largest tracing CTA
+constexpr int kWarpsPerSm = 16;  // FP32 tracing warps per SM, at 128 registers
+constexpr int kRefill = 28;      // idle lanes that a warp refills together
 constexpr double kFaceMargin = 0.02;     // cells
 
 // Inverse-bremsstrahlung modes of the tracer.
@@ -1278,12 +1279,18 @@ __device__ __forceinline__ void reset_cache(CellAheadF2& cc) {
     cc.slot = 0u;
 }
 
-// One-warp CTAs per SM: FP32 at 128 registers (152 with the next cell fetched
-// ahead); FP64 at 168, which holds the
-// polynomials without spilling (256^3 / 4e5 rays: 4.53 ms, against 5.33 ms
-// at 128 registers and 16 warps with 330 B of spill, 4.61 at 10 warps, 4.98 at 8).
+// Threads per CTA of the single-trace kernels. No CTA synchronises; two warps that
+// take neighbouring rays share their cells' lines in L1 (FP32, 256^3 trough / 1e6 rays:
+// 4.40 ms in one-warp CTAs, 4.34 in two, 4.40 in eight; 192^3 / 2e5 1.194, 1.185, 1.230).
+template <class P, bool AHEAD> constexpr int trace_threads() { return sizeof(typename P::R) == 4 && !AHEAD ? 64 : 32; }
+
+// Warps per SM: FP32 16 at 128 registers (12 at 152 with the next cell fetched
+// ahead); FP64 12 at 168, which holds the polynomials without spilling (256^3 /
+// 4e5 rays: 4.53 ms, against 5.33 ms at 128 registers and 16 warps with 330 B of
+// spill, 4.61 at 10 warps, 4.98 at 8).
 template <class P, int INTEG, bool AHEAD> constexpr int trace_min_blocks() {
-    return sizeof(typename P::R) == 4 ? (AHEAD ? 12 : SLOTH_TRACE_MIN_BLOCKS) : (INTEG == INTEG_RK4 ? 8 : 12);
+    const int warps = sizeof(typename P::R) == 4 ? (AHEAD ? 12 : kWarpsPerSm) : (INTEG == INTEG_RK4 ? 8 : 12);
+    return warps * 32 / trace_threads<P, AHEAD>();
 }
 
 // Sum of `v` over the warp, added to *dst by one lane.
