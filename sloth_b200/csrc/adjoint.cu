@@ -1354,9 +1354,8 @@ static int image_forward_impl(const SlothGridDesc* g, const void* grid, const Sl
     // rays in few cells, so that its cell loads and gradient flushes share
     // addresses.
     const int bbits = bucket_bits_for(n);
-    if ((e = cudaMemsetAsync(w.hist, 0, hist_bytes(bbits), s)) != cudaSuccess) return cuda_status(e);
     rc = launch_prepass<typename P::R>(g, p->probing_axis, rays, n, bbits, w.keys, w.hist, w.perm, w.offs, nullptr,
-                                       sms, s);
+                                       nullptr, sms, s);
     if (rc) return rc;
     ImageArgs a;
     fill_image_args(a, g, grid, p, rays, n, w.perm, w.ckpt, w.nsteps);

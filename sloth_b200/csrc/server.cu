@@ -256,7 +256,7 @@ static size_t job_bytes(long long n, const SlothTraceParams* p, int* bbits_out, 
     sz[5] = align256(N * 4);                      // steps
     sz[6] = 256;                                  // total steps
     sz[7] = align256(hist_bytes(bbits));          // histogram
-    sz[8] = align256(N * 4) * 3;                  // keys, perm, bucket offsets
+    sz[8] = align256(N * 4) * 2 + align256(hist_bytes(bbits));   // keys, perm, bucket offsets
     size_t total = 0;
     for (int i = 0; i < 9; ++i) {
         if (parts) parts[i] = total;
@@ -400,10 +400,9 @@ static int admit_one(ServerImpl* s, Job& j) {
     unsigned* offs = reinterpret_cast<unsigned*>(base + parts[8] + 2 * an);
     cudaError_t e = cudaMemcpyAsync(rays, j.rays_src, (size_t)j.n * 6 * 4,
                                     j.rays_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s->admit);
-    if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, hist_bytes(bbits), s->admit);
     int rc = cuda_status(e);
     if (!rc) rc = launch_prepass<float>(&ge->desc, j.p.probing_axis, rays, j.n, bbits, keys, hist, perm, offs,
-                                        j.out.total_steps, s->sms, s->admit);
+                                        j.out.total_steps, nullptr, s->sms, s->admit);
     if (rc) {
         s->arena.release(off, bytes);
         --ge->refs;

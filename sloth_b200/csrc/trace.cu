@@ -103,13 +103,12 @@ static int trace_impl(const SlothGridDesc* g, const void* grid, const SlothTrace
     unsigned* offs = reinterpret_cast<unsigned*>(base + kHeaderBytes + kHistBytes + 2 * an);
 
     const int bbits = bucket_bits_for(n);
-    cudaError_t e = cudaMemsetAsync(base, 0, kHeaderBytes + hist_bytes(bbits), s);
-    if (e != cudaSuccess) return cuda_status(e);
+    cudaError_t e;
     int sms = 148;
     rc = device_sm_count(&sms);
     if (rc) return rc;
     rc = launch_prepass<R>(g, p->probing_axis, reinterpret_cast<const R*>(rays), n, bbits, keys, hist, perm,
-                           offs, out->total_steps, sms, s);
+                           offs, out->total_steps, queue, sms, s);
     if (rc) return rc;
 
     TraceArgs ta;

@@ -42,9 +42,8 @@ class RayServer:
     """Continuous-batching ray-trace server on one GPU.
 
     budget_bytes: HBM admission budget (the arena is allocated up front).
-    tiles_per_step: 1024-ray tiles per iteration (default: four per resident
-    tracer CTA, 8 per SM; shorter iterations pay their launch and retire
-    overhead too often). quantum: tiles per job per round-robin round.
+    tiles_per_step: 1024-ray tiles per iteration (default: 8 per SM; shorter
+    iterations pay their launch and retire overhead too often). quantum: tiles per job per round-robin round.
     """
 
     def __init__(self, budget_bytes: int, *, max_jobs: int = 256, tiles_per_step: Optional[int] = None,

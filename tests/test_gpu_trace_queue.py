@@ -43,7 +43,7 @@ def test_every_ray_once_and_bitwise_the_same(precision, shape, axis, ib):
     keys = ["jones", "phase", "status", "steps"] + (["amp"] if ib else [])
     whole = _trace(most, rays, grid, sched, **kw)
     assert int(whole["total_steps"]) == int(whole["steps"].sum(dtype=torch.int64))
-    for n in (1, 2, 8, 9, 31, 32, 33, 64, 255, 257, 4737, 18944, 18945, 32768, 32769, 148 * 12 * 32, 148 * 12 * 32 + 1,
+    for n in (1, 2, 8, 9, 31, 32, 33, 64, 255, 257, 4737, 18944, 18945, 6144, 6145, 32768, 32769, 148 * 12 * 32, 148 * 12 * 32 + 1,
               65537, most - 33, most - 1):
         part = _trace(n, rays, grid, sched, **kw)
         for k in keys:
