@@ -85,14 +85,22 @@ class DeviceGrid:
 _STAGE_BYTES = 8 << 20
 
 
-def upload(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
+def upload(src: torch.Tensor, dst: torch.Tensor, *, wait: bool = True) -> torch.Tensor:
     """Copy the CPU tensor src into the CUDA tensor dst (same shape and dtype,
-    both contiguous) on the current stream. Pinned memory is copied as it is,
-    without waiting. Pageable memory goes through pinned pieces that the host's threads
+    both contiguous) on the current stream. src may be changed or freed once this
+    returns, pinned or not (numpy arrays over pinned memory, as solve() returns
+    them, too): a pinned source is copied as it is and the call waits for the copy,
+    unless ``wait`` is False, where the caller keeps src unchanged until
+    it has waited for the stream itself. Pageable memory goes through pinned pieces that the host's threads
     fill while the previous piece is copied (the driver's own staging fills
-    them with one thread: 67 MB in 5.6 ms); src may be changed once this returns."""
+    them with one thread: 67 MB in 5.6 ms)."""
     src = src.detach()
-    if src.nbytes <= _STAGE_BYTES // 8 or src.is_pinned():
+    if src.is_pinned():
+        dst.copy_(src, non_blocking=True)
+        if wait:
+            torch.cuda.current_stream(dst.device).synchronize()
+        return dst
+    if src.nbytes <= _STAGE_BYTES // 8:
         return dst.copy_(src, non_blocking=True)
     s, d = src.reshape(-1), dst.view(-1)
     m = _STAGE_BYTES // src.element_size()
@@ -161,7 +169,8 @@ def pack_grid(ne, origin, spacing, omega, *, precision="f32", device=None, strea
         raise ValueError("ne must be a 3-D (nx, ny, nz) array")
     ne = ne.contiguous()
     if ne.device.type != "cuda":
-        ne = upload(ne, torch.empty(ne.shape, dtype=ne.dtype, device=dev))
+        # with the range, its wait at the end covers this copy
+        ne = upload(ne, torch.empty(ne.shape, dtype=ne.dtype, device=dev), wait=not with_range)
     n = tuple(int(k) for k in ne.shape)
     desc = capi.grid_desc(n, origin, spacing)
     rb = 4 if precision == "f32" else 8
@@ -478,7 +487,7 @@ def trace_to_host(grid: DeviceGrid, rays, sched: Schedule, *, want: dict, chunk_
                 if src.device.type == "cuda":
                     st[r].copy_(src[r, a:b], non_blocking=True)
                 else:
-                    upload(src[r, a:b], st[r])
+                    upload(src[r, a:b], st[r], wait=False)   # the lanes are waited for below
             rc = st if src.dtype == dtype else st.to(dtype)
             o = trace(grid, rc, sched, stream=lane, workspace=_lane_workspace(m, dev, li), outputs=outs[li],
                       want_state="state" in want, want_phase="phase" in want, want_amp="amp" in want,

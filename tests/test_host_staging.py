@@ -1,8 +1,12 @@
-"""Staged host copies: around the stage's size, and where no memory can be pinned."""
+"""Staged host copies: around the stage's size, where no memory can be pinned, and
+sources that the caller changes or frees as soon as the call returns."""
+import numpy as np
 import pytest
 import torch
 
 from sloth_b200 import runtime
+from sloth_b200.core import physics
+from sloth_b200.processing import diagnostics
 
 STAGE = runtime._STAGE_BYTES // 4          # float32 elements of one piece
 
@@ -29,3 +33,46 @@ def test_staged_copies_round_trip(monkeypatch, n, fail_at):
     dev = runtime.upload(src, torch.empty(n, device="cuda"))
     assert torch.equal(dev.cpu(), src)
     assert torch.equal(torch.from_numpy(runtime.download(dev)), src)
+
+
+def _busy(ms=20.0):
+    """About `ms` of work on the current stream, so that what follows it is still pending when the host goes on."""
+    a = torch.rand((4096, 4096), device="cuda")
+    a @ a
+    e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    e[0].record()
+    a @ a
+    e[1].record()
+    torch.cuda.synchronize()
+    for _ in range(max(1, int(ms / e[0].elapsed_time(e[1])))):
+        a @ a
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1000, 300_000])                  # below and above a pageable copy's stage
+@pytest.mark.parametrize("stacked", [False, True])
+def test_diagnostic_takes_a_snapshot_of_pinned_rays(n, stacked):
+    """solve() and trace_and_save_depths() return numpy arrays over pinned memory: a
+    Diagnostic holds their values at its construction."""
+    saves = torch.empty((3, 4, n), dtype=torch.float64, pin_memory=True)
+    rf = saves.numpy()
+    rf[:] = np.random.default_rng(n).normal(size=rf.shape) * 1e-3
+    want = rf[-1].copy()
+    _busy()
+    d = diagnostics.Shadowgraphy(rf if stacked else rf[-1], verbose=False)
+    rf[:] = 7.0                                                 # before the queued work can have finished
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(d._rf_in.cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("with_range", [True, False])
+def test_pack_grid_takes_a_snapshot_of_pinned_densities(with_range):
+    ne = torch.rand((60, 61, 62), generator=torch.Generator().manual_seed(1)).pin_memory()
+    kw = dict(precision="f32", layout="values", ne_scale=1.0)
+    ref = runtime.pack_grid(ne.cuda(), (0.0,) * 3, (1e-5,) * 3, physics.omega_of(532e-9), **kw).data.clone()
+    _busy()
+    g = runtime.pack_grid(ne, (0.0,) * 3, (1e-5,) * 3, physics.omega_of(532e-9), with_range=with_range, **kw)
+    ne.fill_(7.0)
+    torch.cuda.synchronize()
+    assert torch.equal(g.data, ref)
