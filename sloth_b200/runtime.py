@@ -185,7 +185,11 @@ def pack_grid(ne, origin, spacing, omega, *, precision="f32", device=None, strea
     geom = (out, desc, precision, float(omega), n, tuple(map(float, origin)), tuple(map(float, spacing)))
     run_on = stream if stream is not None else torch.cuda.current_stream(dev)
     if stream is not None:
-        run_on.wait_stream(torch.cuda.current_stream(dev))   # ne and out belong to the current stream
+        # ne (or its copy made here) and out belong to the current stream: `stream` waits
+        # for them, and their memory for `stream`
+        run_on.wait_stream(torch.cuda.current_stream(dev))
+        ne.record_stream(run_on)
+        out.record_stream(run_on)
     if not with_range:
         if layout == "trace":
             fn = lib.sloth_grid_pack_trace_f32 if rb == 4 else lib.sloth_grid_pack_trace_f64

@@ -70,3 +70,26 @@ def test_pack_on_a_side_stream():
     b = runtime.pack_grid(ne, (0.0,) * 3, (1e-5,) * 3, OMEGA, stream=s)
     torch.cuda.synchronize()
     assert torch.equal(a.data, b.data) and a.ne_max == b.ne_max
+
+
+@pytest.mark.parametrize("source", ["host", "transposed"])
+def test_pack_on_a_side_stream_without_the_range(source):
+    """The call returns before its pack has run: the device copy of ne that it made
+    stays its own although the caller allocates on the current stream at once."""
+    ne = torch.rand((40, 40, 40), generator=torch.Generator().manual_seed(2)) * 1e25
+    ref = runtime.pack_grid(ne, (0.0,) * 3, (1e-5,) * 3, OMEGA).data
+    src = ne if source == "host" else ne.transpose(0, 2).contiguous().cuda().transpose(0, 2)
+    out = torch.empty_like(ref)
+    a = torch.rand((4096, 4096), device="cuda")
+    b = torch.empty_like(a)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        for _ in range(200):                                     # tens of ms
+            torch.mm(a, a, out=b)
+    runtime.pack_grid(src, (0.0,) * 3, (1e-5,) * 3, OMEGA, stream=s, with_range=False, out=out)
+    junk = [torch.full((40, 40, 40), 7e25, device="cuda") for _ in range(4)]
+    assert not s.query()
+    torch.cuda.synchronize()
+    del junk
+    assert torch.equal(out, ref)
