@@ -212,7 +212,9 @@ int sloth_trace_f64(const SlothGridDesc* g, const void* grid, const SlothTracePa
  * (memory released), or a negative SLOTH_ERR_* state if admission failed,
  * or CANCELLED (sloth_server_cancel) from PENDING, RUNNING or DONE.
  * The caller keeps `ne` (needed until the job is admitted, and only if the
- * grid key is not resident) and `rays` valid until the job leaves PENDING.
+ * grid key is not resident) and `rays` valid and unchanged until
+ * sloth_server_inputs_read says yes: the admission's copies run on the device
+ * after the job has left PENDING. It does so before the job is DONE.
  * A handle may be used from several host threads (calls are serialised). */
 typedef struct SlothServer SlothServer;
 
@@ -247,14 +249,24 @@ int sloth_server_destroy(SlothServer* s);
 /* Queues a job. ne (device, float32 or float64 per ne_is_f64, m^-3) is packed
  * when the job is admitted unless grid_key is resident (then ne may be NULL).
  * rays: (6, n) float32, host memory (pinned) if rays_on_host, else device.
- * p as for sloth_trace_f32 (its q_max selects the fast exact paths).
+ * p as for sloth_trace_f32 (its q_max selects the fast exact paths). ne and
+ * rays hold their values when the call is made: the server reads them on streams
+ * of its own that wait for no other (sloth_server_submit_after does).
  * SLOTH_ERR_TOO_LARGE if the job can never fit in the arena. */
 int sloth_server_submit(SlothServer* s, uint64_t grid_key, const SlothGridDesc* g, const void* ne,
                         int ne_is_f64, const SlothTraceParams* p, const float* rays, int rays_on_host,
                         int64_t n, int* job_id);
+/* The same for ne and rays that the work queued on `stream` by now makes: the
+ * job's admission waits for it on the device. */
+int sloth_server_submit_after(SlothServer* s, uint64_t grid_key, const SlothGridDesc* g, const void* ne,
+                              int ne_is_f64, const SlothTraceParams* p, const float* rays, int rays_on_host,
+                              int64_t n, void* stream, int* job_id);
 /* One scheduling step; never blocks on the GPU. */
 int sloth_server_step(SlothServer* s, int* n_running, int* n_pending);
 int sloth_server_job_state(SlothServer* s, int job_id, int* state);
+/* *yes = 1 once the server no longer reads the job's ne and rays (seen by the
+ * latest sloth_server_step; a cancelled or failed job's are not read either). */
+int sloth_server_inputs_read(SlothServer* s, int job_id, int* yes);
 /* Starts the download of a DONE job's outputs into dst (host or device
  * pointers; NULL skips; element types as for sloth_trace_f32, no state);
  * the job's memory is released once the copy has finished (FETCHED). */

@@ -149,8 +149,12 @@ _SIGNATURES = {
     "sloth_server_destroy": (c_int, [c_void_p]),
     "sloth_server_submit": (c_int, [c_void_p, ctypes.c_uint64, POINTER(SlothGridDesc), c_void_p, c_int,
                                     POINTER(SlothTraceParams), c_void_p, c_int, c_int64, POINTER(c_int)]),
+    "sloth_server_submit_after": (c_int, [c_void_p, ctypes.c_uint64, POINTER(SlothGridDesc), c_void_p, c_int,
+                                          POINTER(SlothTraceParams), c_void_p, c_int, c_int64, c_void_p,
+                                          POINTER(c_int)]),
     "sloth_server_step": (c_int, [c_void_p, POINTER(c_int), POINTER(c_int)]),
     "sloth_server_job_state": (c_int, [c_void_p, c_int, POINTER(c_int)]),
+    "sloth_server_inputs_read": (c_int, [c_void_p, c_int, POINTER(c_int)]),
     "sloth_server_fetch": (c_int, [c_void_p, c_int, POINTER(SlothTraceOutputs)]),
     "sloth_server_release": (c_int, [c_void_p, c_int]),
     "sloth_server_stats": (c_int, [c_void_p, POINTER(SlothServerStats)]),

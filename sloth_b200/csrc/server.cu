@@ -190,8 +190,20 @@ struct Job {
     long long last_iter = -1;      // iteration that ran the job's last tiles
     int mode = 0;
     SlothTraceOutputs out{};       // device pointers in the arena
+    cudaEvent_t after = nullptr;   // the caller's work that makes ne and rays (may be null)
+    bool waited = false;           // the admission stream waits for `after`
+    cudaEvent_t ready = nullptr;   // end of the job's admission on the admission stream (its slot's event)
+    bool arrived = false;          // `after` has passed: ne and rays hold their values
+    bool settled = false;          // `ready` has passed: ne and rays are no longer read
     cudaEvent_t fetched = nullptr;
 };
+
+static void destroy_events(Job& j) {
+    for (cudaEvent_t* e : {&j.after, &j.fetched}) {
+        if (*e) cudaEventDestroy(*e);
+        *e = nullptr;
+    }
+}
 
 // Memory of a cancelled RUNNING job, released once the iterations that
 // hold its tiles have finished.
@@ -220,6 +232,8 @@ struct ServerImpl {
     TraceArgs* d_table = nullptr;
     TraceArgs* h_table = nullptr;   // pinned staging of the table rows
     std::vector<int> free_slots;
+    std::vector<cudaEvent_t> slot_ready;   // per slot: end of its job's admission (made at create: making
+                                           // events during a step blocked it for 8 ms now and then)
     std::unordered_map<uint64_t, GridEntry> grids;
     std::unordered_map<int, Job> jobs;
     std::deque<int> pending;
@@ -237,7 +251,6 @@ struct ServerImpl {
     IterSlot it[2];
     cudaStream_t admit = nullptr;   // uploads, packing, pre-pass, table rows
     cudaStream_t copy = nullptr;    // result downloads
-    cudaEvent_t admit_ev = nullptr;
     SlothServerStats stats{};
     std::mutex mu;
 };
@@ -345,6 +358,12 @@ static bool make_room(ServerImpl* s, size_t bytes, size_t* off) {
 
 static int admit_one(ServerImpl* s, Job& j) {
     if (s->free_slots.empty()) return SLOTH_ERR_BUSY;
+    auto wait_inputs = [&]() {   // what follows on the admission stream may read ne and rays
+        if (!j.after || j.waited) return SLOTH_OK;
+        const cudaError_t ev = cudaStreamWaitEvent(s->admit, j.after, 0);
+        j.waited = ev == cudaSuccess;
+        return cuda_status(ev);
+    };
     // grid
     GridEntry* ge = nullptr;
     auto git = s->grids.find(j.grid_key);
@@ -362,8 +381,9 @@ static int admit_one(ServerImpl* s, Job& j) {
         g.off = goff;
         g.bytes = gb;
         const double nc = 3.14207787e-4 * j.p.omega * j.p.omega;
-        int rc = sloth_grid_pack_trace_f32(&j.desc, j.ne, j.ne_is_f64, 1.0 / nc, j.p.ope_ratio2, s->arena.ptr(goff),
-                                           s->admit);
+        int rc = wait_inputs();
+        if (!rc) rc = sloth_grid_pack_trace_f32(&j.desc, j.ne, j.ne_is_f64, 1.0 / nc, j.p.ope_ratio2,
+                                                s->arena.ptr(goff), s->admit);
         if (rc) {
             s->arena.release(goff, gb);
             return rc;
@@ -398,9 +418,11 @@ static int admit_one(ServerImpl* s, Job& j) {
     unsigned* keys = reinterpret_cast<unsigned*>(base + parts[8]);
     unsigned* perm = reinterpret_cast<unsigned*>(base + parts[8] + an);
     unsigned* offs = reinterpret_cast<unsigned*>(base + parts[8] + 2 * an);
-    cudaError_t e = cudaMemcpyAsync(rays, j.rays_src, (size_t)j.n * 6 * 4,
-                                    j.rays_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s->admit);
-    int rc = cuda_status(e);
+    int rc = wait_inputs();
+    cudaError_t e = cudaSuccess;
+    if (!rc) e = cudaMemcpyAsync(rays, j.rays_src, (size_t)j.n * 6 * 4,
+                                 j.rays_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s->admit);
+    if (!rc) rc = cuda_status(e);
     if (!rc) rc = launch_prepass<float>(&ge->desc, j.p.probing_axis, rays, j.n, bbits, keys, hist, perm, offs,
                                         j.out.total_steps, nullptr, s->sms, s->admit);
     if (rc) {
@@ -410,9 +432,11 @@ static int admit_one(ServerImpl* s, Job& j) {
     }
     j.slot = s->free_slots.back();
     s->free_slots.pop_back();
+    j.ready = s->slot_ready[j.slot];
     TraceArgs& ta = s->h_table[j.slot];
     fill_trace_args(ta, &ge->desc, s->arena.ptr(ge->off), &j.p, rays, j.n, &j.out, perm);
     e = cudaMemcpyAsync(s->d_table + j.slot, &ta, sizeof(TraceArgs), cudaMemcpyHostToDevice, s->admit);
+    if (e == cudaSuccess) e = cudaEventRecord(j.ready, s->admit);
     if (e != cudaSuccess) return cuda_status(e);
     j.mode = 2 * trace_mode(&j.p) + (interior_sampling_ok(ta) ? 1 : 0);
     j.tiles_total = (int)((j.n + kTile - 1) / kTile);
@@ -462,6 +486,12 @@ static void retire(ServerImpl* s) {
             s->intervals.erase(it);
         }
     }
+    // admissions end in order
+    for (int id : s->admitted) {
+        Job& j = s->jobs[id];
+        if (!j.settled && cudaEventQuery(j.ready) != cudaSuccess) break;
+        j.settled = true;
+    }
     cudaGetLastError();   // cudaErrorNotReady from the queries
     // jobs whose every tile ran in a finished iteration
     for (size_t i = 0; i < s->admitted.size();) {
@@ -506,6 +536,18 @@ static int launch_iteration(ServerImpl* s) {
             break;
         }
     if (!is || s->admitted.empty()) return SLOTH_OK;
+    // The iteration takes the jobs whose ne and rays are there and waits for their admission on
+    // the device. A job whose caller is late holds up no other; only an empty GPU waits for it.
+    // (Iterations of the jobs alone whose admission has ended: admissions starve behind
+    // one iteration after the other, 9.1e10 ray-steps/s saturated against 9.3e10.)
+    bool arrived = false;
+    for (int id : s->admitted) {
+        Job& j = s->jobs[id];
+        j.arrived = j.arrived || !j.after || cudaEventQuery(j.after) == cudaSuccess;
+        arrived = arrived || (j.arrived && j.tiles_assigned < j.tiles_total);
+    }
+    cudaGetLastError();   // cudaErrorNotReady from the queries
+    cudaEvent_t last_ready = nullptr;   // of the newest job here whose admission has not ended
     // round-robin tiles over admitted jobs
     std::vector<WorkItem> per_mode[kModes];
     const int cap = s->cfg.tiles_per_step;
@@ -516,6 +558,7 @@ static int launch_iteration(ServerImpl* s) {
         any = false;
         for (size_t k = 0; k < s->admitted.size() && taken < cap; ++k) {
             Job& j = s->jobs[s->admitted[(s->rr + k) % s->admitted.size()]];
+            if (arrived && !j.arrived) continue;
             int q = s->cfg.quantum;
             while (q-- > 0 && j.tiles_assigned < j.tiles_total && taken < cap) {
                 per_mode[j.mode].push_back(WorkItem{j.slot, j.tiles_assigned++});
@@ -527,6 +570,10 @@ static int launch_iteration(ServerImpl* s) {
     }
     if (!s->admitted.empty()) s->rr = (s->rr + 1) % s->admitted.size();
     if (taken == 0) return SLOTH_OK;
+    for (int id : s->admitted) {
+        const Job& j = s->jobs[id];
+        if (!j.settled && j.last_iter == iter) last_ready = j.ready;
+    }
     WorkHeader* h = is->h_buf;
     memset(h, 0, sizeof(WorkHeader));
     WorkItem* items = reinterpret_cast<WorkItem*>(h + 1);
@@ -536,8 +583,8 @@ static int launch_iteration(ServerImpl* s) {
         h->offset[m] = at;
         for (const WorkItem& w : per_mode[m]) items[at++] = w;
     }
-    cudaError_t e = cudaEventRecord(s->admit_ev, s->admit);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(is->stream, s->admit_ev, 0);
+    cudaError_t e = cudaSuccess;
+    if (last_ready) e = cudaStreamWaitEvent(is->stream, last_ready, 0);
     if (e == cudaSuccess) e = cudaEventRecord(is->start, is->stream);
     if (e == cudaSuccess) e = cudaGraphLaunch(is->exec, is->stream);
     if (e == cudaSuccess) e = cudaEventRecord(is->done, is->stream);
@@ -621,10 +668,12 @@ int sloth_server_create(const SlothServerConfig* cfg, SlothServer** out) {
                                  true, &allocs)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&s->admit, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&s->copy, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&s->admit_ev, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreate(&s->t0)) != cudaSuccess || (e = cudaEventRecord(s->t0, s->admit)) != cudaSuccess)
         return fail(sloth::cuda_status(e));
     for (int i = cfg->max_jobs - 1; i >= 0; --i) s->free_slots.push_back(i);
+    s->slot_ready.assign((size_t)cfg->max_jobs, nullptr);
+    for (cudaEvent_t& ev : s->slot_ready)
+        if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return fail(sloth::cuda_status(e));
     int blocks[sloth::kModes] = {sloth::resident_blocks<sloth::IB_OFF, 0>(s->sms),
                                  sloth::resident_blocks<sloth::IB_OFF, 1>(s->sms),
                                  sloth::resident_blocks<sloth::IB_SUBCRITICAL, 0>(s->sms),
@@ -653,8 +702,9 @@ int sloth_server_destroy(SlothServer* srv) {
         if (is.stream) cudaStreamSynchronize(is.stream);
     if (s->admit) cudaStreamSynchronize(s->admit);
     if (s->copy) cudaStreamSynchronize(s->copy);
-    for (auto& kv : s->jobs)
-        if (kv.second.fetched) cudaEventDestroy(kv.second.fetched);
+    for (auto& kv : s->jobs) sloth::destroy_events(kv.second);
+    for (cudaEvent_t ev : s->slot_ready)
+        if (ev) cudaEventDestroy(ev);
     for (auto& is : s->it) {
         if (is.exec) cudaGraphExecDestroy(is.exec);
         if (is.done) cudaEventDestroy(is.done);
@@ -663,7 +713,6 @@ int sloth_server_destroy(SlothServer* srv) {
         if (is.d_buf) cudaFree(is.d_buf);
         if (is.stream) cudaStreamDestroy(is.stream);
     }
-    if (s->admit_ev) cudaEventDestroy(s->admit_ev);
     if (s->t0) cudaEventDestroy(s->t0);
     if (s->admit) cudaStreamDestroy(s->admit);
     if (s->copy) cudaStreamDestroy(s->copy);
@@ -675,9 +724,9 @@ int sloth_server_destroy(SlothServer* srv) {
     return SLOTH_OK;
 }
 
-int sloth_server_submit(SlothServer* srv, uint64_t grid_key, const SlothGridDesc* g, const void* ne,
-                        int ne_is_f64, const SlothTraceParams* p, const float* rays, int rays_on_host,
-                        int64_t n, int* job_id) {
+static int submit_job(SlothServer* srv, uint64_t grid_key, const SlothGridDesc* g, const void* ne, int ne_is_f64,
+                      const SlothTraceParams* p, const float* rays, int rays_on_host, int64_t n, bool ordered,
+                      void* stream, int* job_id) {
     if (!srv || !p || !job_id) return SLOTH_ERR_NULL_POINTER;
     int rc = sloth::check_trace_params(g, p, n);
     if (rc) return rc;
@@ -705,12 +754,32 @@ int sloth_server_submit(SlothServer* srv, uint64_t grid_key, const SlothGridDesc
     if (n == 0) {
         j.state = sloth::JOB_FETCHED;
     } else {
+        if (ordered) {
+            cudaError_t e = cudaEventCreateWithFlags(&j.after, cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaEventRecord(j.after, (cudaStream_t)stream);
+            if (e != cudaSuccess) {
+                sloth::destroy_events(j);
+                return sloth::cuda_status(e);
+            }
+        }
         s->pending.push_back(j.id);
     }
     s->jobs[j.id] = j;
     ++s->stats.jobs_submitted;
     *job_id = j.id;
     return SLOTH_OK;
+}
+
+int sloth_server_submit(SlothServer* srv, uint64_t grid_key, const SlothGridDesc* g, const void* ne,
+                        int ne_is_f64, const SlothTraceParams* p, const float* rays, int rays_on_host,
+                        int64_t n, int* job_id) {
+    return submit_job(srv, grid_key, g, ne, ne_is_f64, p, rays, rays_on_host, n, false, nullptr, job_id);
+}
+
+int sloth_server_submit_after(SlothServer* srv, uint64_t grid_key, const SlothGridDesc* g, const void* ne,
+                              int ne_is_f64, const SlothTraceParams* p, const float* rays, int rays_on_host,
+                              int64_t n, void* stream, int* job_id) {
+    return submit_job(srv, grid_key, g, ne, ne_is_f64, p, rays, rays_on_host, n, true, stream, job_id);
 }
 
 int sloth_server_step(SlothServer* srv, int* n_running, int* n_pending) {
@@ -743,6 +812,17 @@ int sloth_server_job_state(SlothServer* srv, int job_id, int* state) {
     auto it = s->jobs.find(job_id);
     if (it == s->jobs.end()) return SLOTH_ERR_NOT_FOUND;
     *state = it->second.state;
+    return SLOTH_OK;
+}
+
+int sloth_server_inputs_read(SlothServer* srv, int job_id, int* yes) {
+    if (!srv || !yes) return SLOTH_ERR_NULL_POINTER;
+    ServerImpl* s = &srv->impl;
+    std::lock_guard<std::mutex> lock(s->mu);
+    auto it = s->jobs.find(job_id);
+    if (it == s->jobs.end()) return SLOTH_ERR_NOT_FOUND;
+    const sloth::Job& j = it->second;
+    *yes = j.state != sloth::JOB_PENDING && (j.settled || j.state != sloth::JOB_ADMITTED);
     return SLOTH_OK;
 }
 
@@ -782,7 +862,7 @@ int sloth_server_release(SlothServer* srv, int job_id) {
     if (j.state == sloth::JOB_PENDING || j.state == sloth::JOB_ADMITTED || j.state == sloth::JOB_FETCHING)
         return SLOTH_ERR_BUSY;
     if (j.state == sloth::JOB_DONE) sloth::free_job_memory(s, j);
-    if (j.fetched) cudaEventDestroy(j.fetched);
+    sloth::destroy_events(j);
     s->jobs.erase(it);
     return SLOTH_OK;
 }
@@ -803,6 +883,8 @@ int sloth_server_cancel(SlothServer* srv, int job_id) {
                 }
             break;
         case sloth::JOB_ADMITTED: {
+            // ne and rays may go once this returns
+            if (!j.settled) cudaEventSynchronize(j.ready);
             // no further tiles; the memory waits for the iterations that hold
             // the tiles already handed out (last_iter), which may still run
             for (size_t i = 0; i < s->admitted.size(); ++i)

@@ -32,7 +32,7 @@ class Job:
     inv_brems: bool
     arrival: float = 0.0
     state: int = capi.SLOTH_JOB_PENDING
-    keep: list = field(default_factory=list)      # buffers the server reads until admission
+    keep: list = field(default_factory=list)      # buffers the server reads until the job's admission has ended
     out: Optional[dict] = None                    # pinned host results once fetched
     done_at: Optional[float] = None
     request: Optional[object] = None              # the stream request it serves (replay)
@@ -82,7 +82,8 @@ class RayServer:
                arrival: Optional[float] = None) -> Job:
         """Queue a trace of `rays` ((6, N) float32, CUDA or pinned CPU) through
         the grid `grid_key`. `ne` (m^-3, CUDA) is needed unless the key is
-        resident; the server packs it on admission. The rays are traced to
+        resident; the server packs it on admission. Both are read once the work
+        queued on the current stream has run; `inputs_read` says when they no longer are. The rays are traced to
         c*t = sqrt(8)*depth (depth defaults to the grid's extent along the
         probing axis); with `detector_plane` the final rays are projected to it."""
         omega = physics.omega_of(lwl)
@@ -124,9 +125,12 @@ class RayServer:
             ne_ptr = ne.data_ptr()
             ne_f64 = int(ne.dtype == torch.float64)
         jid = ctypes.c_int(0)
-        capi.check(self.lib.sloth_server_submit(self.handle, ctypes.c_uint64(grid_key), desc, ne_ptr, ne_f64, p,
-                                                rays.data_ptr(), int(on_host), n_rays, ctypes.byref(jid)),
-                   "sloth_server_submit")
+        # the server's streams wait for no other: the job's admission waits for
+        # what the current stream has yet to do for ne and rays
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        capi.check(self.lib.sloth_server_submit_after(self.handle, ctypes.c_uint64(grid_key), desc, ne_ptr, ne_f64, p,
+                                                      rays.data_ptr(), int(on_host), n_rays, stream,
+                                                      ctypes.byref(jid)), "sloth_server_submit_after")
         job = Job(jid.value, n_rays, sched.n_saves, bool(inv_brems),
                   arrival=time.perf_counter() if arrival is None else arrival, keep=[ne, rays])
         if n_rays == 0:
@@ -148,9 +152,17 @@ class RayServer:
         job.state = st.value
         if st.value < 0:
             raise capi.SlothError(st.value, f"job {job.id}")
-        if st.value != capi.SLOTH_JOB_PENDING:
+        if job.keep and st.value != capi.SLOTH_JOB_PENDING and self.inputs_read(job):
             job.keep = []
         return st.value
+
+    def inputs_read(self, job: Job) -> bool:
+        """Whether the server has read the job's ne and rays (before that the
+        caller must not change them; the server holds references to them)."""
+        yes = ctypes.c_int(0)
+        capi.check(self.lib.sloth_server_inputs_read(self.handle, job.id, ctypes.byref(yes)),
+                   "sloth_server_inputs_read")
+        return bool(yes.value)
 
     @staticmethod
     def _host_outputs(job: Job) -> dict:

@@ -140,6 +140,95 @@ def test_dense_job_in_the_mix_with_fast_path_jobs():
     _same(outs[-1], {k: v.cpu() for k, v in direct.items()})
 
 
+def _busy():
+    """Tens of milliseconds of work on the current stream."""
+    a = torch.rand((4096, 4096), device="cuda")
+    b = torch.empty_like(a)
+    for _ in range(200):
+        torch.mm(a, a, out=b)
+
+
+@pytest.mark.parametrize("running", [False, True])
+def test_rays_and_density_that_the_callers_stream_still_makes(running):
+    """A job reads its rays and a new grid's density once the caller's stream has made
+    them, also while other jobs run, which go on meanwhile."""
+    n, nrays = 48, 50_000
+    h = L / (n - 1)
+    key = serving.grid_key("kolmogorov", n, 0)
+    fields = {key: serving.field_for("kolmogorov", n, 0, L=L)}
+    rays = workloads.gaussian_beam(nrays, waist=2e-3, L=L, seed=5, jitter=1e-3, device="cuda")
+    ref = _direct(fields, "kolmogorov", n, rays)
+    kw = dict(lwl=LWL, detector_plane=L / 2, Te=20.0, Z=1.0)
+    with serving.RayServer(2 << 30) as srv:
+        slab = {serving.grid_key("sinusoid", 64, 0): serving.field_for("sinusoid", 64, 0, L=L)}
+        srv.run_until_done([_submit(srv, slab, "sinusoid", 64, 100_000, 0)[0]])   # kernels are loaded
+        others = [_submit(srv, slab, "sinusoid", 64, 100_000, i)[0] for i in (1, 2)] if running else []
+        ne, late = torch.zeros_like(fields[key]), torch.zeros_like(rays)
+        srv._qmax[key] = _qrange(fields[key])            # submit itself would wait for a new key's range
+        torch.cuda.synchronize()
+        _busy()
+        ne.copy_(fields[key])
+        late.copy_(rays)
+        job = srv.submit(key, ne, (-L / 2,) * 3, (h,) * 3, (n,) * 3, late, inv_brems=True, **kw)
+        res = srv.run_until_done([job] + others)
+        _same(res[job.id], ref)
+
+
+def _qrange(ne):
+    nc = physics.critical_density(physics.omega_of(LWL))
+    return max(float(ne.max()) / nc, 0.0) * (1 + 1e-6), min(float(ne.min()) / nc, 0.0) * (1 + 1e-6)
+
+
+@pytest.mark.parametrize("how", ["changed", "freed"])
+def test_rays_may_go_once_they_are_read(how):
+    """The server holds the rays until its copy of them has run on the device (here a large
+    grid's pack stands before it): the caller may change them once inputs_read says
+    so, and may drop them, and allocate anew, at any time."""
+    n, nrays = 400, 50_000
+    h = L / (n - 1)
+    key = serving.grid_key("sinusoid", n, 0)
+    fields = {key: serving.field_for("sinusoid", n, 0, L=L)}
+    rays = workloads.gaussian_beam(nrays, waist=2e-3, L=L, seed=6, device="cuda")
+    ref = _direct(fields, "sinusoid", n, rays)
+    with serving.RayServer(4 << 30) as srv:
+        srv._qmax[key] = _qrange(fields[key])
+        torch.cuda.synchronize()
+        job = srv.submit(key, fields[key], (-L / 2,) * 3, (h,) * 3, (n,) * 3, rays, lwl=LWL, detector_plane=L / 2)
+        if how == "changed":
+            while not srv.inputs_read(job):
+                srv.step()
+            rays.fill_(1.0)
+        else:
+            del rays
+            while srv.state(job) == _capi.SLOTH_JOB_PENDING:
+                srv.step()
+            junk = [torch.ones((6, nrays), device="cuda") for _ in range(4)]
+        _same(srv.run_until_done([job])[job.id], ref)
+        assert not job.keep
+        if how == "freed":
+            del junk
+
+
+def test_cancel_while_the_admission_waits_for_the_caller():
+    n = 48
+    key = serving.grid_key("sinusoid", n, 0)
+    fields = {key: serving.field_for("sinusoid", n, 0, L=L)}
+    with serving.RayServer(1 << 30) as srv:
+        first, _ = _submit(srv, fields, "sinusoid", n, 20_000, 1)
+        srv.run_until_done([first])
+        torch.cuda.synchronize()
+        _busy()
+        job, _ = _submit(srv, fields, "sinusoid", n, 20_000, 2)
+        srv.step()
+        assert not srv.inputs_read(job)
+        srv.cancel(job)
+        assert srv.inputs_read(job)
+        srv.release(job)
+        again, rays = _submit(srv, fields, "sinusoid", n, 20_000, 3)
+        _same(srv.run_until_done([again])[again.id], _direct(fields, "sinusoid", n, rays))
+        assert srv.stats()["cancelled_pending_free"] == 0
+
+
 def test_job_without_rays_in_the_mix():
     """A job of zero rays finishes at once with empty results of the usual
     shapes; the job submitted beside it is unaffected."""
