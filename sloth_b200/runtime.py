@@ -83,15 +83,42 @@ class DeviceGrid:
 
 
 _STAGE_BYTES = 8 << 20
+_STAGE_PIECES = 8
 
 
-def upload(src: torch.Tensor, dst: torch.Tensor, *, wait: bool = True) -> torch.Tensor:
+class _Staging:
+    """Pinned pieces that pageable memory passes through: at most _STAGE_PIECES of
+    _STAGE_BYTES, each used again once its last copy is done (so a host that is faster
+    than the stream waits, and page-locks no more than these)."""
+
+    def __init__(self):
+        self._pieces = []                  # (piece, event behind its last copy), oldest first
+
+    def take(self, nbytes: int):
+        """A piece of nbytes or more (uint8) that no copy uses, or None where the host has no memory to pin."""
+        if len(self._pieces) < _STAGE_PIECES and not (self._pieces and self._pieces[0][1].query()):
+            piece = _pinned(nbytes, torch.uint8)
+            if piece is not None or not self._pieces:
+                return piece
+        piece, done = self._pieces.pop(0)
+        done.synchronize()
+        return piece if piece.numel() >= nbytes else _pinned(nbytes, torch.uint8)
+
+    def used(self, piece: torch.Tensor, stream):
+        """The copy queued last on `stream` uses piece."""
+        done = torch.cuda.Event()
+        done.record(stream)
+        self._pieces.append((piece, done))
+
+
+def upload(src: torch.Tensor, dst: torch.Tensor, *, wait: bool = True, staging: Optional[_Staging] = None) -> torch.Tensor:
     """Copy the CPU tensor src into the CUDA tensor dst (same shape and dtype,
     both contiguous) on the current stream. src may be changed or freed once this
     returns, pinned or not (numpy arrays over pinned memory, as solve() returns
     them, too): a pinned source is copied as it is and the call waits for the copy,
     unless ``wait`` is False, where the caller keeps src unchanged until
-    it has waited for the stream itself. Pageable memory goes through pinned pieces that the host's threads
+    it has waited for the stream itself. Pageable memory goes through the pinned pieces of
+    ``staging`` (the call's own by default), which the host's threads
     fill while the previous piece is copied (the driver's own staging fills
     them with one thread: 67 MB in 5.6 ms)."""
     src = src.detach()
@@ -102,16 +129,18 @@ def upload(src: torch.Tensor, dst: torch.Tensor, *, wait: bool = True) -> torch.
         return dst
     if src.nbytes <= _STAGE_BYTES // 8:
         return dst.copy_(src, non_blocking=True)
+    staging = staging or _Staging()
     s, d = src.reshape(-1), dst.view(-1)
     m = _STAGE_BYTES // src.element_size()
     for a in range(0, s.numel(), m):
-        # the caching host allocator reuses a piece once its copy is done
-        piece = _pinned(min(m, s.numel() - a), s.dtype)
+        part = s[a:a + m]
+        piece = staging.take(part.nbytes)
         if piece is None:
             d[a:].copy_(s[a:], non_blocking=True)
             break
-        piece.copy_(s[a:a + m])
-        d[a:a + m].copy_(piece, non_blocking=True)
+        piece[:part.nbytes].view(s.dtype).copy_(part)
+        d[a:a + m].copy_(piece[:part.nbytes].view(s.dtype), non_blocking=True)
+        staging.used(piece, torch.cuda.current_stream(dst.device))
     return dst
 
 
@@ -476,6 +505,7 @@ def trace_to_host(grid: DeviceGrid, rays, sched: Schedule, *, want: dict, chunk_
         lane.wait_event(ready)
     outs = ({}, {})
     stage = [None, None]
+    staging = _Staging()                   # one for the call: the host may run ahead of the lanes
     t0 = time.perf_counter()
     for c in range(n_chunks):
         a, b = bounds[c], bounds[c + 1]
@@ -491,7 +521,7 @@ def trace_to_host(grid: DeviceGrid, rays, sched: Schedule, *, want: dict, chunk_
                 if src.device.type == "cuda":
                     st[r].copy_(src[r, a:b], non_blocking=True)
                 else:
-                    upload(src[r, a:b], st[r], wait=False)   # the lanes are waited for below
+                    upload(src[r, a:b], st[r], wait=False, staging=staging)   # the lanes are waited for below
             rc = st if src.dtype == dtype else st.to(dtype)
             o = trace(grid, rc, sched, stream=lane, workspace=_lane_workspace(m, dev, li), outputs=outs[li],
                       want_state="state" in want, want_phase="phase" in want, want_amp="amp" in want,
