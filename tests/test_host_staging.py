@@ -116,3 +116,32 @@ def test_a_chunked_trace_of_pageable_rays_pins_no_more_pieces(monkeypatch):
     assert len(pieces.at) <= runtime._STAGE_PIECES
     whole = runtime.trace(grid, torch.from_numpy(rays).float().cuda(), sched)
     assert torch.equal(torch.from_numpy(got["jones"]), whole["jones"].cpu()) and steps == int(whole["total_steps"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [STAGE // 8 + 1, STAGE, STAGE + 1, 4 * STAGE + 3])
+@pytest.mark.parametrize("strided", [False, True])
+def test_results_in_ordinary_memory(monkeypatch, n, strided):
+    monkeypatch.setattr(runtime, "_PINNED_RESULT_BYTES", 0)
+    t = torch.rand((n, 2), device="cuda")[:, 0] if strided else torch.rand(n, device="cuda")
+    got = runtime.download(t)
+    assert not torch.from_numpy(got).is_pinned()
+    assert torch.equal(torch.from_numpy(got), t.cpu())
+
+
+@pytest.mark.gpu
+def test_callers_hold_a_bounded_amount_of_pinned_results():
+    t = torch.rand(runtime._PINNED_RESULT_BYTES // 4 // 3 + 1, device="cuda")         # two fit, three do not
+    want = t.cpu()
+    is_pinned = lambda a: torch.from_numpy(a).is_pinned()  # noqa: E731
+    before = runtime._pinned_results
+    assert before == 0, "results of other tests are gone"
+    kept = [runtime.download(t) for _ in range(4)]
+    assert [is_pinned(a) for a in kept] == [True, True, False, False]
+    assert all(torch.equal(torch.from_numpy(a), want) for a in kept)
+    part = kept[0][5:]
+    del kept
+    assert runtime._pinned_results == t.nbytes           # the view holds its array
+    del part
+    assert runtime._pinned_results == 0
+    assert is_pinned(runtime.download(t))
