@@ -11,6 +11,7 @@ import math
 import struct
 import threading
 import weakref
+from collections import OrderedDict
 from dataclasses import dataclass
 from typing import Optional
 
@@ -298,6 +299,10 @@ def sample(grid: DeviceGrid, points, *, stream=None) -> torch.Tensor:
     n = pts.shape[1]
     out = torch.empty((4, n), dtype=grid.data.dtype, device=grid.data.device)
     fn = capi.load().sloth_sample_f32 if grid.precision == "f32" else capi.load().sloth_sample_f64
+    if stream is not None and stream != torch.cuda.current_stream(grid.data.device):
+        stream.wait_stream(torch.cuda.current_stream(grid.data.device))   # pts and out are made on the current stream
+        pts.record_stream(stream)
+        out.record_stream(stream)
     capi.check(fn(grid.desc, capi.ptr(grid.data), capi.ptr(pts), n, capi.ptr(out), _stream_ptr(stream)),
                "sloth_sample")
     return out
@@ -341,16 +346,27 @@ def schedule_times(tau_saves, spacing) -> Schedule:
     return Schedule(d / m, 0, m, int(tau_saves.size))
 
 
-_ws_cache: dict = {}
+_ws_cache: OrderedDict = OrderedDict()     # (device, stream, thread) -> workspace, oldest first
+_ws_lock = threading.Lock()
+_WS_KEPT = 8
 
 
-def _workspace(n: int, device) -> torch.Tensor:
+def _workspace(n: int, dev, stream) -> torch.Tensor:
+    """The scratch memory of a trace of n rays on `stream`: one per stream and thread,
+    because a trace's kernels must not meet another's in it (two threads' launches on one stream may
+    alternate). The _WS_KEPT used last are kept; they belong to their stream, so one that is
+    given back is reused behind the kernels that still use it."""
     need = int(capi.load().sloth_trace_workspace_bytes(n))
-    key = (str(device),)
-    t = _ws_cache.get(key)
+    key = (str(dev), int(stream.cuda_stream), threading.get_ident())
+    with _ws_lock:
+        t = _ws_cache.pop(key, None)
     if t is None or t.numel() < need:
-        t = torch.empty(need, dtype=torch.uint8, device=device)
+        with torch.cuda.stream(stream):
+            t = torch.empty(need, dtype=torch.uint8, device=dev)
+    with _ws_lock:
         _ws_cache[key] = t
+        while len(_ws_cache) > _WS_KEPT:
+            _ws_cache.popitem(last=False)
     return t
 
 
@@ -380,8 +396,10 @@ def trace(grid: DeviceGrid, rays: torch.Tensor, sched: Schedule, *, axis=2, proj
     if grid.layout != "trace":
         raise ValueError("the tracers read grids packed with layout='trace'")
     dtype = torch.float32 if grid.precision == "f32" else torch.float64
+    own = []                               # tensors made here
     if rays.dtype != dtype or rays.device != grid.data.device or not rays.is_contiguous():
         rays = rays.to(device=grid.data.device, dtype=dtype).contiguous()
+        own.append(rays)
     if rays.dim() != 2 or rays.shape[0] != 6:
         raise ValueError("rays must have shape (6, N)")
     n = int(rays.shape[1])
@@ -399,6 +417,7 @@ def trace(grid: DeviceGrid, rays: torch.Tensor, sched: Schedule, *, axis=2, proj
         if t is None or tuple(t.shape) != tuple(shape) or t.dtype != dt:
             t = torch.empty(shape, dtype=dt, device=dev)
             o[key] = t
+            own.append(t)
         return t
 
     jones = buf("jones", (S, 4, n), dtype)
@@ -437,10 +456,16 @@ def trace(grid: DeviceGrid, rays: torch.Tensor, sched: Schedule, *, axis=2, proj
     if events is not None:
         out.trace_event_begin = int(events[0].cuda_event)
         out.trace_event_end = int(events[1].cuda_event)
-    ws = workspace if workspace is not None else _workspace(n, dev)
+    run_on = stream if stream is not None else torch.cuda.current_stream(dev)
+    if stream is not None and own and stream != torch.cuda.current_stream(dev):
+        # made on the current stream, used on `stream`
+        stream.wait_stream(torch.cuda.current_stream(dev))
+        for t in own:
+            t.record_stream(stream)
+    ws = workspace if workspace is not None else _workspace(n, dev, run_on)
     fn = capi.load().sloth_trace_f32 if grid.precision == "f32" else capi.load().sloth_trace_f64
     capi.check(fn(grid.desc, capi.ptr(grid.data), p, capi.ptr(rays), n, out, capi.ptr(ws), ws.numel(),
-                  _stream_ptr(stream)), "sloth_trace")
+                  _stream_ptr(run_on)), "sloth_trace")
     return o
 
 
@@ -455,16 +480,6 @@ def _lanes(dev):
         lanes = (torch.cuda.Stream(dev), torch.cuda.Stream(dev))
         _lane_cache[key] = lanes
     return lanes
-
-
-def _lane_workspace(n: int, dev, lane: int) -> torch.Tensor:
-    need = int(capi.load().sloth_trace_workspace_bytes(n))
-    key = (str(dev), "lane", lane)
-    t = _ws_cache.get(key)
-    if t is None or t.numel() < need:
-        t = torch.empty(need, dtype=torch.uint8, device=dev)
-        _ws_cache[key] = t
-    return t
 
 
 STREAM_CHUNK_RAYS = 1 << 24
@@ -574,7 +589,7 @@ def trace_to_host(grid: DeviceGrid, rays, sched: Schedule, *, want: dict, chunk_
                 else:
                     upload(src[r, a:b], st[r], wait=False, staging=staging)   # the lanes are waited for below
             rc = st if src.dtype == dtype else st.to(dtype)
-            o = trace(grid, rc, sched, stream=lane, workspace=_lane_workspace(m, dev, li), outputs=outs[li],
+            o = trace(grid, rc, sched, stream=lane, outputs=outs[li],
                       want_state="state" in want, want_phase="phase" in want, want_amp="amp" in want,
                       want_status="status" in want, want_steps="steps" in want, **kw)
             for k, h in host.items():
