@@ -56,8 +56,8 @@ constexpr int kAdjThreads = 32;
 constexpr int kAdjStateWords = 5;
 // Two FP32 builds of the backward: 16 warps per SM (128 registers) when as
 // many segment buffers fit an SM's shared memory (on B200, 228 KB per SM and
-// 1 KB reserved per CTA: checkpoints at most every 20 steps), 12 (168
-// registers) otherwise. FP64 runs 8. The FP32 forward runs 24 (80 registers).
+// 1 KB reserved per CTA: checkpoints at most every 21 steps), 12 otherwise
+// (room for 168 registers a thread, of which it takes 148). FP64 runs 8. The FP32 forward runs 24 (80 registers).
 template <class P> constexpr int adj_fwd_min_blocks() { return sizeof(typename P::R) == 4 ? 24 : 12; }
 constexpr int kMaxCkptEvery = 32;
 constexpr int kMaxTaps = 65;          // 2 * 4 * sigma + 1 pixels at sigma <= 8
@@ -189,9 +189,9 @@ __device__ __forceinline__ bool locate(const GridGeo& g, const typename P::R (&h
     return true;
 }
 
-// FP32: the gradient channels as two polynomial pairs, (q, dq/du) and
-// (dq/dv, dq/dw), in the float4 voxel's own register pairs, evaluated with
-// sm_100's paired FP32 instructions (q is carried along at no cost).
+// FP32: the gradient channels as a scalar polynomial, dq/du, and a pair of
+// them, (dq/dv, dq/dw), evaluated with sm_100's paired FP32 instructions. (As the
+// pair (q, dq/du), q would be carried along on the FMA pipe.)
 struct GradCellF2 {
     unsigned base;
     float t0[8];      // dq/du
@@ -905,7 +905,7 @@ __device__ __forceinline__ void splat_adjoint(const ImageArgs& a, double pa, dou
 
 // The tracer's interior-step test on the model state: inside the grid, and
 // the prediction p + w at least kFaceMargin inside on every axis. With every
-// stage acceleration below kInteriorAccel, all four stage points of the step
+// stage acceleration below kInteriorAccel, all stage points of the step
 // are then inside, and locate needs no grid test.
 template <class P>
 __device__ __forceinline__ bool model_interior(const ImageArgs& a, const MState<P>& r) {

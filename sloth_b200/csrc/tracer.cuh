@@ -40,15 +40,6 @@
 
 #include "common.cuh"
 
-#ifndef SLOTH_TRACE_THREADS
-#define SLOTH_TRACE_THREADS 32
-#endif
-#ifndef SLOTH_TRACE_MIN_BLOCKS
-#define SLOTH_TRACE_MIN_BLOCKS 16
-#endif
-#ifndef SLOTH_REFILL
-#define SLOTH_REFILL 28
-#endif
 namespace sloth {
 
 constexpr int kThreads = 64;     // threads of the largest tracing CTA
@@ -612,13 +603,8 @@ __device__ __forceinline__ void sample_f2(const TraceArgs& a, float hx, float lx
     out.g0 = r0.y;
     out.g1 = r1.x;
     out.g2 = r1.y;
-    if constexpr (IB == IB_SUBCRITICAL) {
-        out.k = kappa_eval(fx, fyz.x, fyz.y);   // cl_lo / ope2^2 is in tau_scale
-    } else if constexpr (IB == IB_GENERAL) {
-        out.k = kappa_eval(fx, fyz.x, fyz.y);
-    } else {
-        out.k = 0.0f;
-    }
+    if constexpr (IB != IB_OFF) out.k = kappa_eval(fx, fyz.x, fyz.y);   // sub-critical: cl_lo / ope2^2 is in tau_scale
+    else out.k = 0.0f;
 }
 
 // s + x with the compensation c (AccF::add on a pair)
@@ -1171,7 +1157,7 @@ struct RangeQueue {
 // 1e6 rays with 6 mm beams (many side exits): 132.6 and - ms refilled one by one,
 // 117.1 and 5.21 at 8 idle lanes, 107.1 and 5.13 at 16, 105.4 and 5.13 at 24,
 // 104.7 and 5.20 at 30, 105.0 and 5.43 at 32. Nothing else synchronises: a CTA
-// is one warp, and no warp waits for another one's rays. (Tiles of 1024 rays,
+// is one or two warps, and no warp waits for another one's rays. (Tiles of 1024 rays,
 // sorted and traced by CTAs of eight warps that met at each tile's end, took
 // 110.7 ms; and a small trace's tiles kept most SMs idle: 1e4 rays through
 // 128^3 took 180 us in the kernel on 40 CTAs, 113 us on 313.)
