@@ -8,10 +8,26 @@ namespace sloth {
 // fetches the next cell ahead while its 12 warps per SM hold all the rays at once,
 // the 16-warp one above. With few warps a step waits for its cell (long scoreboard
 // a third of it); with 16 the load and store pipe has no room for the ring's
-// extra copies. Measured without / with: 3e3 rays, 128^3 127 / 103 us; 1e4 129 / 105;
-// 192^3 turbulent, 3e4 526 / 470, 5.6e4 575 / 523, 7.2e4 627 / 682; along x, 2e4 rays
-// 679 / 536 us; 512^3, 1e7 rays 105 / 119 ms.
-constexpr int kAheadWarps = 12;
+// extra copies. Measured, time of the 16-warp build over the other's, turbulent and slab
+// fields, along x, y and z (the two transverse strides differ: the cells that a ray along
+// z crosses share lines):
+//   rays               3e3        1e4        3e4        5e4        5.7e4 (12 warps)  7.2e4 (16-warp build)
+//   512^3          1.0 .. 1.64 1.1 .. 1.60 1.1 .. 1.43 1.0 .. 1.26 1.0 .. 1.27      0.94 .. 1.31
+//   256^3          1.1 .. 1.64 1.0 .. 1.60 1.1 .. 1.37 1.0 .. 1.26 1.0 .. 1.27      0.84 .. 1.09
+//   192^3          1.0 .. 1.19 1.1 .. 1.32 1.1 .. 1.14 1.0 .. 1.12 1.0 .. 1.13      0.85 .. 0.94
+//   128^3          1.0 .. 1.13 1.0 .. 1.13 1.0 .. 1.03 .97 .. 1.00 .94 .. 1.03      0.83 .. 1.04
+//   64^3           1.0 .. 1.10 1.0 .. 1.03 .95 .. 1.02 .93 .. 1.01 .90 .. 1.02      0.81 .. 0.98
+// A grid of up to 6 MB spreads over the SMs' L1s (40 KB each), where a cell comes
+// soon enough once every scheduler has more than one warp: there four warps per SM end
+// the build's range (64^3 turbulent, 3e4 and 5.7e4 rays 4 and 10 % faster so, the slab
+// within 2 %; at 80^3 to 128^3 the turbulent field would gain 3 to 5 % and the slab lose as much).
+// 512^3, 1e7 rays: 105 ms against 119.
+constexpr int kAheadWarps = 12, kAheadWarpsL1 = 4;
+constexpr long long kL1GridBytes = 6LL << 20;
+static bool fetch_ahead(const TraceArgs& ta, int sms) {
+    const long long bytes = 16LL * ta.geo.n[0] * ta.geo.n[1] * ta.geo.n[2];
+    return ta.n <= (long long)sms * (bytes <= kL1GridBytes ? kAheadWarpsL1 : kAheadWarps) * 32;
+}
 // Rays of a warp's first take: 32, or as few as kSpreadMin as long as that gives
 // each of an SM's four schedulers one warp (fewer rays, fewer cells that the warp waits
 // for: FP64, 5e3 rays 597 -> 529 us; 1e4 rays, 128^3 107 -> 105). More, smaller warps
@@ -68,7 +84,7 @@ template <class P, int IB>
 static int launch_trace(const TraceArgs& ta, int sms, cudaStream_t s, int fast, int integ) {
     if (integ == INTEG_RK4) return launch_trace_i<P, IB, INTEG_RK4>(ta, sms, s, fast);
     if constexpr (sizeof(typename P::R) == 4)
-        if (ta.n <= (long long)sms * kAheadWarps * 32) return launch_trace_i<P, IB, INTEG_RKN, true>(ta, sms, s, fast);
+        if (fetch_ahead(ta, sms)) return launch_trace_i<P, IB, INTEG_RKN, true>(ta, sms, s, fast);
     return launch_trace_i<P, IB, INTEG_RKN>(ta, sms, s, fast);
 }
 

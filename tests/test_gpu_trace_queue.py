@@ -27,14 +27,16 @@ def _trace(n_rays, rays, grid, sched, **kw):
 @pytest.mark.parametrize("precision", ["f32", "f64"])
 @pytest.mark.parametrize("shape,axis,ib,integ", [((20, 33, 24), 2, True, "rkn"), ((2, 2, 40), 2, False, "rkn"),
                                                  ((31, 18, 27), 0, True, "rkn"), ((19, 22, 30), 1, False, "rkn"),
-                                                 ((20, 33, 24), 2, True, "rk4")])
+                                                 ((20, 33, 24), 2, True, "rk4"),
+                                                 ((90, 80, 81), 1, True, "rkn")])      # a grid of more than 6 MB
 def test_every_ray_once_and_bitwise_the_same(precision, shape, axis, ib, integ):
     h = tuple(L / (k - 1) for k in shape)
     g = torch.Generator().manual_seed(3)
     ne = (torch.rand(shape, generator=g) * 2e25).float()
     grid = runtime.pack_grid(ne, (-L / 2,) * 3, h, physics.omega_of(532e-9), precision=precision)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    ahead = sms * 12 * 32                # the largest trace of the build that fetches ahead
+    # the largest trace of the build that fetches ahead
+    ahead = sms * 32 * (12 if 16 * shape[0] * shape[1] * shape[2] > 6 << 20 else 4)
     most = sms * 16 * 32 + 33            # the warps at 16 per SM, and one more warp's worth
     assert most - 33 > ahead             # so the builds are compared
     rays = workloads.gaussian_beam(most, waist=3e-3, L=L, jitter=5e-2, seed=2, device="cuda", dtype=torch.float64)
