@@ -192,6 +192,7 @@ struct Job {
     SlothTraceOutputs out{};       // device pointers in the arena
     cudaEvent_t after = nullptr;   // the caller's work that makes ne and rays (may be null)
     bool waited = false;           // the admission stream waits for `after`
+    bool packing = false;          // a pack of ne is queued there (the job's own memory may not have fitted yet)
     cudaEvent_t ready = nullptr;   // end of the job's admission on the admission stream (its slot's event)
     bool arrived = false;          // `after` has passed: ne and rays hold their values
     bool settled = false;          // `ready` has passed: ne and rays are no longer read
@@ -388,6 +389,7 @@ static int admit_one(ServerImpl* s, Job& j) {
             s->arena.release(goff, gb);
             return rc;
         }
+        j.packing = true;
         ++s->stats.grid_packs;
         ge = &(s->grids[j.grid_key] = g);
     }
@@ -876,6 +878,7 @@ int sloth_server_cancel(SlothServer* srv, int job_id) {
     sloth::Job& j = it->second;
     switch (j.state) {
         case sloth::JOB_PENDING:
+            if (j.packing) cudaStreamSynchronize(s->admit);   // ne may go once this returns
             for (auto q = s->pending.begin(); q != s->pending.end(); ++q)
                 if (*q == job_id) {
                     s->pending.erase(q);

@@ -114,7 +114,8 @@ class _Staging:
         self._pieces.append((piece, done))
 
 
-def upload(src: torch.Tensor, dst: torch.Tensor, *, wait: bool = True, staging: Optional[_Staging] = None) -> torch.Tensor:
+def upload(src: torch.Tensor, dst: torch.Tensor, *, wait: bool = True,
+           staging: Optional[_Staging] = None) -> torch.Tensor:
     """Copy the CPU tensor src into the CUDA tensor dst (same shape and dtype,
     both contiguous) on the current stream. src may be changed or freed once this
     returns, pinned or not (numpy arrays over pinned memory, as solve() returns

@@ -229,6 +229,37 @@ def test_cancel_while_the_admission_waits_for_the_caller():
         assert srv.stats()["cancelled_pending_free"] == 0
 
 
+def test_cancel_of_a_job_whose_grid_is_being_packed():
+    """A pending job whose grid went in but whose own memory did not fit: once it is
+    cancelled the caller may change ne, and the resident grid is the one it gave."""
+    n, nrays = 400, 2_000_000
+    fields = {serving.grid_key("sinusoid", m, 0): serving.field_for("sinusoid", m, 0, L=L) for m in (32, n)}
+    key = serving.grid_key("sinusoid", n, 0)
+    h = L / (n - 1)
+    few = workloads.gaussian_beam(5000, waist=2e-3, L=L, seed=3, device="cuda")
+    ref = _direct(fields, "sinusoid", n, few)
+    with serving.RayServer(16 * (n ** 3 + 32 ** 3) + 100 * nrays) as srv:
+        side = torch.cuda.Stream()
+        srv._qmax[key] = _qrange(fields[key])
+        # the kernels are loaded: a first launch would wait for the GPU
+        torch.empty_like(fields[key]).fill_(3e25)
+        srv.run_until_done([_submit(srv, fields, "sinusoid", 32, 5000, 0)[0]])
+        first, _ = _submit(srv, fields, "sinusoid", 32, nrays, 1)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):                    # a late caller (0.1 s on one SM): the pack stands behind it
+            torch.cuda._sleep(200_000_000)
+            job, _ = _submit(srv, fields, "sinusoid", n, nrays, 2)
+        srv.step()
+        assert srv.state(first) == _capi.SLOTH_JOB_RUNNING and srv.state(job) == _capi.SLOTH_JOB_PENDING
+        assert srv.stats()["grid_packs"] == 2
+        srv.cancel(job)
+        fields[key].fill_(3e25)
+        srv.release(job)
+        srv.run_until_done([first])
+        again = srv.submit(key, None, (-L / 2,) * 3, (h,) * 3, (n,) * 3, few, lwl=LWL, detector_plane=L / 2)
+        _same(srv.run_until_done([again])[again.id], ref)
+
+
 def test_job_without_rays_in_the_mix():
     """A job of zero rays finishes at once with empty results of the usual
     shapes; the job submitted beside it is unaffected."""
