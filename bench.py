@@ -715,7 +715,7 @@ def run_sloth(args):
                                  "logical_gather_gbs": gather_gbs},
                          "note": "achieved = ray-steps/s x FP32 lane-operations per ray-step (ncu instruction "
                                  "mix: scalar FFMA/FADD/FMUL + 2 x paired FFMA2/FADD2/FMUL2); the trace is bound "
-                                 "by its FP32 pipes, not memory: DRAM traffic (traffic, from ncu) is ~1.5 B per "
+                                 "by its FP32 pipes, not memory: DRAM traffic (traffic, from ncu) is ~1.3 B per "
                                  "ray-step against 384 logical gather bytes, which a register cell cache and L1 "
                                  "serve"},
             "cpu_baseline": cpu,
