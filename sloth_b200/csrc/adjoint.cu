@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(256) accel_bound_kernel(const void* __restrict
 // ckpt_every steps and the final state. The warp's rays run in step, so between
 // checkpoints (and for as many steps as every live ray's run allows) the steps
 // follow each other in a uniform loop. Bound by instruction issue (71 %, FMA pipe 64 %):
-// 128^3, 1e6 rays, 400 steps in 2.94 ms (1.33e11 ray-steps/s), 185 instructions a
+// 128^3, 1e6 rays, 400 steps in 2.92 ms (1.34e11 ray-steps/s), 183 instructions a
 // ray-step; 3.26 ms and 235 before the paired step, the scalar dq/du polynomial and
 // this loop.
 template <class P>
