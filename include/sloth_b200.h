@@ -200,8 +200,8 @@ int sloth_trace_f64(const SlothGridDesc* g, const void* grid, const SlothTracePa
  * stream of trace jobs of different grids and ray counts by continuous
  * batching: one device arena of budget_bytes (allocated at create) holds the
  * packed grids -- an LRU cache keyed by the caller's 64-bit grid key -- and
- * each admitted job's rays, sort workspace and outputs. Jobs are admitted in
- * submission order as memory and job-table slots free up. Every
+ * each admitted job's rays, sort workspace and outputs. Jobs whose inputs are
+ * there are admitted in submission order as memory and job-table slots free up. Every
  * sloth_server_step() retires finished work, admits waiting jobs, and
  * launches one iteration -- a captured CUDA graph running the FP32 tracer's
  * persistent kernels over tiles handed out round-robin to all admitted jobs
@@ -257,7 +257,7 @@ int sloth_server_submit(SlothServer* s, uint64_t grid_key, const SlothGridDesc* 
                         int ne_is_f64, const SlothTraceParams* p, const float* rays, int rays_on_host,
                         int64_t n, int* job_id);
 /* The same for ne and rays that the work queued on `stream` by now makes: the
- * job's admission waits for it on the device. */
+ * job is admitted once that work has run, other jobs before it if theirs has. */
 int sloth_server_submit_after(SlothServer* s, uint64_t grid_key, const SlothGridDesc* g, const void* ne,
                               int ne_is_f64, const SlothTraceParams* p, const float* rays, int rays_on_host,
                               int64_t n, void* stream, int* job_id);

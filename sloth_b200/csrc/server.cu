@@ -3,8 +3,8 @@
 //
 // Memory: one device arena of `budget_bytes` (a single cudaMalloc at
 // create) holds the packed grids (an LRU cache keyed by the caller) and each
-// admitted job's rays, sort workspace and outputs. A job is admitted, in
-// arrival order, when its grid and its memory fit and a job-table slot is
+// admitted job's rays, sort workspace and outputs. A job whose ne and rays are
+// there is admitted, in arrival order, when its grid and its memory fit and a job-table slot is
 // free; otherwise it waits. Idle grids (no admitted job) are evicted LRU to
 // make room.
 //
@@ -191,10 +191,9 @@ struct Job {
     int mode = 0;
     SlothTraceOutputs out{};       // device pointers in the arena
     cudaEvent_t after = nullptr;   // the caller's work that makes ne and rays (may be null)
-    bool waited = false;           // the admission stream waits for `after`
-    bool packing = false;          // a pack of ne is queued there (the job's own memory may not have fitted yet)
-    cudaEvent_t ready = nullptr;   // end of the job's admission on the admission stream (its slot's event)
     bool arrived = false;          // `after` has passed: ne and rays hold their values
+    bool packing = false;          // a pack of ne is queued (the job's own memory may not have fitted yet)
+    cudaEvent_t ready = nullptr;   // end of the job's admission on the admission stream (its slot's event)
     bool settled = false;          // `ready` has passed: ne and rays are no longer read
     cudaEvent_t fetched = nullptr;
 };
@@ -359,12 +358,6 @@ static bool make_room(ServerImpl* s, size_t bytes, size_t* off) {
 
 static int admit_one(ServerImpl* s, Job& j) {
     if (s->free_slots.empty()) return SLOTH_ERR_BUSY;
-    auto wait_inputs = [&]() {   // what follows on the admission stream may read ne and rays
-        if (!j.after || j.waited) return SLOTH_OK;
-        const cudaError_t ev = cudaStreamWaitEvent(s->admit, j.after, 0);
-        j.waited = ev == cudaSuccess;
-        return cuda_status(ev);
-    };
     // grid
     GridEntry* ge = nullptr;
     auto git = s->grids.find(j.grid_key);
@@ -382,9 +375,8 @@ static int admit_one(ServerImpl* s, Job& j) {
         g.off = goff;
         g.bytes = gb;
         const double nc = 3.14207787e-4 * j.p.omega * j.p.omega;
-        int rc = wait_inputs();
-        if (!rc) rc = sloth_grid_pack_trace_f32(&j.desc, j.ne, j.ne_is_f64, 1.0 / nc, j.p.ope_ratio2,
-                                                s->arena.ptr(goff), s->admit);
+        int rc = sloth_grid_pack_trace_f32(&j.desc, j.ne, j.ne_is_f64, 1.0 / nc, j.p.ope_ratio2, s->arena.ptr(goff),
+                                           s->admit);
         if (rc) {
             s->arena.release(goff, gb);
             return rc;
@@ -420,11 +412,9 @@ static int admit_one(ServerImpl* s, Job& j) {
     unsigned* keys = reinterpret_cast<unsigned*>(base + parts[8]);
     unsigned* perm = reinterpret_cast<unsigned*>(base + parts[8] + an);
     unsigned* offs = reinterpret_cast<unsigned*>(base + parts[8] + 2 * an);
-    int rc = wait_inputs();
-    cudaError_t e = cudaSuccess;
-    if (!rc) e = cudaMemcpyAsync(rays, j.rays_src, (size_t)j.n * 6 * 4,
-                                 j.rays_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s->admit);
-    if (!rc) rc = cuda_status(e);
+    cudaError_t e = cudaMemcpyAsync(rays, j.rays_src, (size_t)j.n * 6 * 4,
+                                    j.rays_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s->admit);
+    int rc = cuda_status(e);
     if (!rc) rc = launch_prepass<float>(&ge->desc, j.p.probing_axis, rays, j.n, bbits, keys, hist, perm, offs,
                                         j.out.total_steps, nullptr, s->sms, s->admit);
     if (rc) {
@@ -530,6 +520,21 @@ static void retire(ServerImpl* s) {
     cudaGetLastError();
 }
 
+// The next job to admit: the first of the queue whose ne and rays are there (of its
+// first kLook: a long queue of late callers is not searched on every step); a late
+// caller holds up no other. pending.end() if there is none.
+constexpr int kLook = 16;
+static std::deque<int>::iterator next_pending(ServerImpl* s) {
+    auto it = s->pending.begin();
+    for (int k = 0; k < kLook && it != s->pending.end(); ++k, ++it) {
+        Job& j = s->jobs[*it];
+        j.arrived = j.arrived || !j.after || cudaEventQuery(j.after) == cudaSuccess;
+        if (j.arrived) return it;
+    }
+    cudaGetLastError();   // cudaErrorNotReady from the queries
+    return s->pending.end();
+}
+
 static int launch_iteration(ServerImpl* s) {
     IterSlot* is = nullptr;
     for (IterSlot& c : s->it)
@@ -538,18 +543,6 @@ static int launch_iteration(ServerImpl* s) {
             break;
         }
     if (!is || s->admitted.empty()) return SLOTH_OK;
-    // The iteration takes the jobs whose ne and rays are there and waits for their admission on
-    // the device. A job whose caller is late holds up no other; only an empty GPU waits for it.
-    // (Iterations of the jobs alone whose admission has ended: admissions starve behind
-    // one iteration after the other, 9.1e10 ray-steps/s saturated against 9.3e10.)
-    bool arrived = false;
-    for (int id : s->admitted) {
-        Job& j = s->jobs[id];
-        j.arrived = j.arrived || !j.after || cudaEventQuery(j.after) == cudaSuccess;
-        arrived = arrived || (j.arrived && j.tiles_assigned < j.tiles_total);
-    }
-    cudaGetLastError();   // cudaErrorNotReady from the queries
-    cudaEvent_t last_ready = nullptr;   // of the newest job here whose admission has not ended
     // round-robin tiles over admitted jobs
     std::vector<WorkItem> per_mode[kModes];
     const int cap = s->cfg.tiles_per_step;
@@ -560,7 +553,6 @@ static int launch_iteration(ServerImpl* s) {
         any = false;
         for (size_t k = 0; k < s->admitted.size() && taken < cap; ++k) {
             Job& j = s->jobs[s->admitted[(s->rr + k) % s->admitted.size()]];
-            if (arrived && !j.arrived) continue;
             int q = s->cfg.quantum;
             while (q-- > 0 && j.tiles_assigned < j.tiles_total && taken < cap) {
                 per_mode[j.mode].push_back(WorkItem{j.slot, j.tiles_assigned++});
@@ -572,6 +564,10 @@ static int launch_iteration(ServerImpl* s) {
     }
     if (!s->admitted.empty()) s->rr = (s->rr + 1) % s->admitted.size();
     if (taken == 0) return SLOTH_OK;
+    // The iteration waits for its jobs' admission on the device. (Iterations of the jobs alone
+    // whose admission has ended: admissions starve behind one iteration after the
+    // other, 9.1e10 ray-steps/s saturated against 9.2e10.)
+    cudaEvent_t last_ready = nullptr;   // of the newest job here whose admission has not ended
     for (int id : s->admitted) {
         const Job& j = s->jobs[id];
         if (!j.settled && j.last_iter == iter) last_ready = j.ready;
@@ -757,8 +753,12 @@ static int submit_job(SlothServer* srv, uint64_t grid_key, const SlothGridDesc* 
         j.state = sloth::JOB_FETCHED;
     } else {
         if (ordered) {
-            cudaError_t e = cudaEventCreateWithFlags(&j.after, cudaEventDisableTiming);
-            if (e == cudaSuccess) e = cudaEventRecord(j.after, (cudaStream_t)stream);
+            cudaError_t e = cudaStreamQuery((cudaStream_t)stream);   // an idle stream has made them
+            if (e == cudaErrorNotReady) {
+                cudaGetLastError();
+                e = cudaEventCreateWithFlags(&j.after, cudaEventDisableTiming);
+                if (e == cudaSuccess) e = cudaEventRecord(j.after, (cudaStream_t)stream);
+            }
             if (e != cudaSuccess) {
                 sloth::destroy_events(j);
                 return sloth::cuda_status(e);
@@ -789,11 +789,11 @@ int sloth_server_step(SlothServer* srv, int* n_running, int* n_pending) {
     ServerImpl* s = &srv->impl;
     std::lock_guard<std::mutex> lock(s->mu);
     sloth::retire(s);
-    while (!s->pending.empty()) {
-        sloth::Job& j = s->jobs[s->pending.front()];
+    for (auto it = sloth::next_pending(s); it != s->pending.end(); it = sloth::next_pending(s)) {
+        sloth::Job& j = s->jobs[*it];
         const int rc = sloth::admit_one(s, j);
         if (rc == SLOTH_ERR_BUSY || rc == SLOTH_ERR_OUT_OF_MEMORY) break;   // wait for memory / slots
-        s->pending.pop_front();
+        s->pending.erase(it);
         if (rc) {
             j.state = rc;   // negative: failed
             ++s->stats.jobs_failed;

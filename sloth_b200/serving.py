@@ -2,7 +2,7 @@
 
 ``RayServer`` wraps ``sloth_server_*`` (include/sloth_b200.h): grids stay
 resident in an HBM arena sized by the admission budget (LRU by grid key),
-jobs are admitted in arrival order as memory and slots free up, and each
+jobs whose inputs are there are admitted in arrival order as memory and slots free up, and each
 ``step()`` launches one graph-captured iteration of the persistent FP32
 tracer over tiles of all admitted jobs. ``replay()`` drives a server with a
 timed request stream (seeded Poisson arrivals) and reports p50/p99 latency
@@ -125,8 +125,8 @@ class RayServer:
             ne_ptr = ne.data_ptr()
             ne_f64 = int(ne.dtype == torch.float64)
         jid = ctypes.c_int(0)
-        # the server's streams wait for no other: the job's admission waits for
-        # what the current stream has yet to do for ne and rays
+        # the server's streams wait for no other: the job is admitted when the current
+        # stream has done what it has yet to do for ne and rays
         stream = torch.cuda.current_stream(self.device).cuda_stream
         capi.check(self.lib.sloth_server_submit_after(self.handle, ctypes.c_uint64(grid_key), desc, ne_ptr, ne_f64, p,
                                                       rays.data_ptr(), int(on_host), n_rays, stream,

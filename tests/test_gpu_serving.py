@@ -238,26 +238,44 @@ def test_cancel_of_a_job_whose_grid_is_being_packed():
     h = L / (n - 1)
     few = workloads.gaussian_beam(5000, waist=2e-3, L=L, seed=3, device="cuda")
     ref = _direct(fields, "sinusoid", n, few)
+    other = torch.full((n, n, n), 3e25).pin_memory()
     with serving.RayServer(16 * (n ** 3 + 32 ** 3) + 100 * nrays) as srv:
-        side = torch.cuda.Stream()
         srv._qmax[key] = _qrange(fields[key])
-        # the kernels are loaded: a first launch would wait for the GPU
-        torch.empty_like(fields[key]).fill_(3e25)
-        srv.run_until_done([_submit(srv, fields, "sinusoid", 32, 5000, 0)[0]])
+        srv.run_until_done([_submit(srv, fields, "sinusoid", 32, 5000, 0)[0]])    # the kernels are loaded
         first, _ = _submit(srv, fields, "sinusoid", 32, nrays, 1)
+        job, _ = _submit(srv, fields, "sinusoid", n, nrays, 2)
         torch.cuda.synchronize()
-        with torch.cuda.stream(side):                    # a late caller (0.1 s on one SM): the pack stands behind it
-            torch.cuda._sleep(200_000_000)
-            job, _ = _submit(srv, fields, "sinusoid", n, nrays, 2)
+        with torch.cuda.stream(torch.cuda.Stream()):     # the pack waits for room
+            _busy()
         srv.step()
         assert srv.state(first) == _capi.SLOTH_JOB_RUNNING and srv.state(job) == _capi.SLOTH_JOB_PENDING
         assert srv.stats()["grid_packs"] == 2
         srv.cancel(job)
-        fields[key].fill_(3e25)
+        fields[key].copy_(other, non_blocking=True)      # a copy engine's work: it needs no room
+        torch.cuda.synchronize()
         srv.release(job)
         srv.run_until_done([first])
         again = srv.submit(key, None, (-L / 2,) * 3, (h,) * 3, (n,) * 3, few, lwl=LWL, detector_plane=L / 2)
         _same(srv.run_until_done([again])[again.id], ref)
+
+
+def test_a_late_caller_holds_up_no_other():
+    """Jobs submitted after one whose rays are still being made are admitted, traced and
+    fetched before it."""
+    n = 48
+    fields = {serving.grid_key("sinusoid", n, 0): serving.field_for("sinusoid", n, 0, L=L)}
+    with serving.RayServer(1 << 30) as srv:
+        srv.run_until_done([_submit(srv, fields, "sinusoid", n, 20_000, 0)[0]])
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda._sleep(400_000_000)               # 0.2 s on one SM
+            late, late_rays = _submit(srv, fields, "sinusoid", n, 20_000, 1)
+        jobs = [_submit(srv, fields, "sinusoid", n, 20_000, k) for k in (2, 3)]
+        res = srv.run_until_done([j for j, _ in jobs])
+        assert srv.state(late) == _capi.SLOTH_JOB_PENDING
+        for j, rays in jobs:
+            _same(res[j.id], _direct(fields, "sinusoid", n, rays))
+        _same(srv.run_until_done([late])[late.id], _direct(fields, "sinusoid", n, late_rays))
 
 
 def test_job_without_rays_in_the_mix():
