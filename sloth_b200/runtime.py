@@ -358,14 +358,17 @@ def _workspace(n: int, dev, stream) -> torch.Tensor:
     alternate). The _WS_KEPT used last are kept; they belong to their stream, so one that is
     given back is reused behind the kernels that still use it."""
     need = int(capi.load().sloth_trace_workspace_bytes(n))
-    key = (str(dev), int(stream.cuda_stream), threading.get_ident())
+    key = (dev.index, int(stream.cuda_stream), threading.get_ident())
     with _ws_lock:
-        t = _ws_cache.pop(key, None)
-    if t is None or t.numel() < need:
-        with torch.cuda.stream(stream):
-            t = torch.empty(need, dtype=torch.uint8, device=dev)
+        t = _ws_cache.get(key)
+        if t is not None and t.numel() >= need:
+            _ws_cache.move_to_end(key)
+            return t
+    with torch.cuda.stream(stream):
+        t = torch.empty(need, dtype=torch.uint8, device=dev)
     with _ws_lock:
         _ws_cache[key] = t
+        _ws_cache.move_to_end(key)
         while len(_ws_cache) > _WS_KEPT:
             _ws_cache.popitem(last=False)
     return t

@@ -1,5 +1,7 @@
 """Staged host copies: around the stage's size, where no memory can be pinned, and
 sources that the caller changes or frees as soon as the call returns."""
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -134,8 +136,8 @@ def test_callers_hold_a_bounded_amount_of_pinned_results():
     t = torch.rand(runtime._PINNED_RESULT_BYTES // 4 // 3 + 1, device="cuda")         # two fit, three do not
     want = t.cpu()
     is_pinned = lambda a: torch.from_numpy(a).is_pinned()  # noqa: E731
-    before = runtime._pinned_results
-    assert before == 0, "results of other tests are gone"
+    gc.collect()
+    assert runtime._pinned_results == 0, "results of other tests are gone"
     kept = [runtime.download(t) for _ in range(4)]
     assert [is_pinned(a) for a in kept] == [True, True, False, False]
     assert all(torch.equal(torch.from_numpy(a), want) for a in kept)
