@@ -91,27 +91,35 @@ _STAGE_PIECES = 8
 
 class _Staging:
     """Pinned pieces that pageable memory passes through: at most _STAGE_PIECES of
-    _STAGE_BYTES, each used again once its last copy is done (so a host that is faster
-    than the stream waits, and page-locks no more than these)."""
+    _STAGE_BYTES with copies in flight, so that a host that is faster than its streams waits and
+    page-locks no more than these. The caching allocator hands a piece out again once
+    its copy is done; an event behind every few pieces holds the host back."""
 
     def __init__(self):
-        self._pieces = []                  # (piece, event behind its last copy), oldest first
+        self._marks = []                   # (event, pieces before it since the last one), oldest first
+        self._open, self._stream = 0, None   # pieces behind the last mark, and their stream
+
+    def _mark(self):
+        if self._open:
+            done = torch.cuda.Event()
+            done.record(self._stream)
+            self._marks.append((done, self._open))
+            self._open = 0
 
     def take(self, nbytes: int):
-        """A piece of nbytes or more (uint8) that no copy uses, or None where the host has no memory to pin."""
-        if len(self._pieces) < _STAGE_PIECES and not (self._pieces and self._pieces[0][1].query()):
-            piece = _pinned(nbytes, torch.uint8)
-            if piece is not None or not self._pieces:
-                return piece
-        piece, done = self._pieces.pop(0)
-        done.synchronize()
-        return piece if piece.numel() >= nbytes else _pinned(nbytes, torch.uint8)
+        """A piece of nbytes (uint8), or None where the host has no memory to pin."""
+        while self._open + sum(k for _, k in self._marks) >= _STAGE_PIECES:
+            self._marks.pop(0)[0].synchronize()
+        return _pinned(nbytes, torch.uint8)
 
-    def used(self, piece: torch.Tensor, stream):
-        """The copy queued last on `stream` uses piece."""
-        done = torch.cuda.Event()
-        done.record(stream)
-        self._pieces.append((piece, done))
+    def used(self, stream):
+        """The copy queued last on `stream` uses the piece taken last."""
+        if stream != self._stream:
+            self._mark()
+            self._stream = stream
+        self._open += 1
+        if 2 * self._open >= _STAGE_PIECES:
+            self._mark()
 
 
 def upload(src: torch.Tensor, dst: torch.Tensor, *, wait: bool = True,
@@ -138,13 +146,15 @@ def upload(src: torch.Tensor, dst: torch.Tensor, *, wait: bool = True,
     m = _STAGE_BYTES // src.element_size()
     for a in range(0, s.numel(), m):
         part = s[a:a + m]
+        piece = None                       # the last one goes back first
         piece = staging.take(part.nbytes)
         if piece is None:
             d[a:].copy_(s[a:], non_blocking=True)
             break
-        piece[:part.nbytes].view(s.dtype).copy_(part)
-        d[a:a + m].copy_(piece[:part.nbytes].view(s.dtype), non_blocking=True)
-        staging.used(piece, torch.cuda.current_stream(dst.device))
+        piece = piece.view(s.dtype)
+        piece.copy_(part)
+        d[a:a + m].copy_(piece, non_blocking=True)
+        staging.used(torch.cuda.current_stream(dst.device))
     return dst
 
 
