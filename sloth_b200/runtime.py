@@ -172,33 +172,48 @@ def _pinned(shape, dtype):
 # page-lock, and pay for, a new block each time (52 ms), so beyond this results are ordinary memory.
 _PINNED_RESULT_BYTES = 256 << 20
 _pinned_results = 0
-_pinned_lock = threading.RLock()           # reentrant: a finalizer may run anywhere
+_pinned_lock = threading.RLock()           # reentrant: a result may go while it is held
+_pinned_refs: dict = {}                    # the references whose callbacks give the bytes back
 
 
-def _hold_pinned(nbytes: int) -> bool:
+class _Held(weakref.ref):
+    """Reference to a pinned result that gives its bytes back when it goes (weakref.finalize
+    does as much in 10 us more)."""
+    __slots__ = ("nbytes",)
+
+
+def _release(ref):
     global _pinned_results
     with _pinned_lock:
-        if nbytes > 0 and _pinned_results + nbytes > _PINNED_RESULT_BYTES:
-            return False
+        _pinned_results -= ref.nbytes
+        _pinned_refs.pop(id(ref), None)
+
+
+def _hold(result: np.ndarray, nbytes: int):
+    """Count a pinned result for as long as it (or a view of it) lives."""
+    global _pinned_results
+    ref = _Held(result, _release)
+    ref.nbytes = nbytes
+    with _pinned_lock:
         _pinned_results += nbytes
-        return True
+        _pinned_refs[id(ref)] = ref
 
 
 def download(t: torch.Tensor) -> np.ndarray:
     """The CUDA tensor t as a numpy array: in pinned memory when it is large and
     callers hold no more than _PINNED_RESULT_BYTES of such results, otherwise in ordinary memory."""
-    if t.nbytes <= _STAGE_BYTES // 8:
+    nbytes = t.nbytes
+    if nbytes <= _STAGE_BYTES // 8:
         return t.cpu().numpy()
     stream = torch.cuda.current_stream(t.device)
-    if _hold_pinned(t.nbytes):
+    if _pinned_results + nbytes <= _PINNED_RESULT_BYTES:
         h = _pinned(t.shape, t.dtype)
         if h is not None:
             h.copy_(t, non_blocking=True)
-            stream.synchronize()
             out = h.numpy()
-            weakref.finalize(out, _hold_pinned, -t.nbytes)     # views of it keep it alive
+            _hold(out, nbytes)             # while the copy runs
+            stream.synchronize()
             return out
-        _hold_pinned(-t.nbytes)
     s = t.detach().reshape(-1)
     host = torch.empty(t.shape, dtype=t.dtype)
     d = host.view(-1)
