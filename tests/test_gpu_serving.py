@@ -278,6 +278,29 @@ def test_a_late_caller_holds_up_no_other():
         _same(srv.run_until_done([late])[late.id], _direct(fields, "sinusoid", n, late_rays))
 
 
+@pytest.mark.parametrize("entry", ["sloth_server_submit", "sloth_server_submit_after"])
+def test_host_rays_through_either_entry(entry):
+    """Pinned host rays that are there already, with and without a stream to wait for."""
+    n = 48
+    fields = {serving.grid_key("sinusoid", n, 0): serving.field_for("sinusoid", n, 0, L=L)}
+    key, h = serving.grid_key("sinusoid", n, 0), L / (n - 1)
+    rays = workloads.gaussian_beam(20_001, waist=2e-3, L=L, seed=4)
+    torch.cuda.synchronize()
+    with serving.RayServer(1 << 30) as srv:
+        lib = srv.lib
+
+        class Entry:                                     # the library with the other submit in place
+            def __getattr__(self, name):
+                if name == "sloth_server_submit_after" and entry == "sloth_server_submit":
+                    return lambda *a: lib.sloth_server_submit(*a[:-2], a[-1])
+                return getattr(lib, name)
+        srv.lib = Entry()
+        job = srv.submit(key, fields[key], (-L / 2,) * 3, (h,) * 3, (n,) * 3, rays.pin_memory(), lwl=LWL,
+                         detector_plane=L / 2)
+        _same(srv.run_until_done([job])[job.id], _direct(fields, "sinusoid", n, rays.cuda()))
+        srv.lib = lib
+
+
 def test_job_without_rays_in_the_mix():
     """A job of zero rays finishes at once with empty results of the usual
     shapes; the job submitted beside it is unaffected."""
