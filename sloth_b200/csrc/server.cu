@@ -198,13 +198,6 @@ struct Job {
     cudaEvent_t fetched = nullptr;
 };
 
-static void destroy_events(Job& j) {
-    for (cudaEvent_t* e : {&j.after, &j.fetched}) {
-        if (*e) cudaEventDestroy(*e);
-        *e = nullptr;
-    }
-}
-
 // Memory of a cancelled RUNNING job, released once the iterations that
 // hold its tiles have finished.
 struct DeferredFree {
@@ -232,6 +225,7 @@ struct ServerImpl {
     TraceArgs* d_table = nullptr;
     TraceArgs* h_table = nullptr;   // pinned staging of the table rows
     std::vector<int> free_slots;
+    std::vector<cudaEvent_t> spare_events; // of jobs that have gone, for the next ones
     std::vector<cudaEvent_t> slot_ready;   // per slot: end of its job's admission (made at create: making
                                            // events during a step blocked it for 8 ms now and then)
     std::unordered_map<uint64_t, GridEntry> grids;
@@ -254,6 +248,20 @@ struct ServerImpl {
     SlothServerStats stats{};
     std::mutex mu;
 };
+
+static cudaError_t take_event(ServerImpl* s, cudaEvent_t* e) {
+    if (s->spare_events.empty()) return cudaEventCreateWithFlags(e, cudaEventDisableTiming);
+    *e = s->spare_events.back();
+    s->spare_events.pop_back();
+    return cudaSuccess;
+}
+
+static void give_events(ServerImpl* s, Job& j) {
+    for (cudaEvent_t* e : {&j.after, &j.fetched}) {
+        if (*e) s->spare_events.push_back(*e);
+        *e = nullptr;
+    }
+}
 
 static size_t job_bytes(long long n, const SlothTraceParams* p, int* bbits_out, size_t* parts) {
     const size_t N = (size_t)(n > 0 ? n : 1);
@@ -700,7 +708,8 @@ int sloth_server_destroy(SlothServer* srv) {
         if (is.stream) cudaStreamSynchronize(is.stream);
     if (s->admit) cudaStreamSynchronize(s->admit);
     if (s->copy) cudaStreamSynchronize(s->copy);
-    for (auto& kv : s->jobs) sloth::destroy_events(kv.second);
+    for (auto& kv : s->jobs) sloth::give_events(s, kv.second);
+    for (cudaEvent_t ev : s->spare_events) cudaEventDestroy(ev);
     for (cudaEvent_t ev : s->slot_ready)
         if (ev) cudaEventDestroy(ev);
     for (auto& is : s->it) {
@@ -753,14 +762,10 @@ static int submit_job(SlothServer* srv, uint64_t grid_key, const SlothGridDesc* 
         j.state = sloth::JOB_FETCHED;
     } else {
         if (ordered) {
-            cudaError_t e = cudaStreamQuery((cudaStream_t)stream);   // an idle stream has made them
-            if (e == cudaErrorNotReady) {
-                cudaGetLastError();
-                e = cudaEventCreateWithFlags(&j.after, cudaEventDisableTiming);
-                if (e == cudaSuccess) e = cudaEventRecord(j.after, (cudaStream_t)stream);
-            }
+            cudaError_t e = sloth::take_event(s, &j.after);
+            if (e == cudaSuccess) e = cudaEventRecord(j.after, (cudaStream_t)stream);
             if (e != cudaSuccess) {
-                sloth::destroy_events(j);
+                sloth::give_events(s, j);
                 return sloth::cuda_status(e);
             }
         }
@@ -847,7 +852,7 @@ int sloth_server_fetch(SlothServer* srv, int job_id, const SlothTraceOutputs* ds
     cp(dst->status, j.out.status, N);
     cp(dst->steps, j.out.steps, N * 4);
     cp(dst->total_steps, j.out.total_steps, 8);
-    if (e == cudaSuccess && !j.fetched) e = cudaEventCreateWithFlags(&j.fetched, cudaEventDisableTiming);
+    if (e == cudaSuccess && !j.fetched) e = sloth::take_event(s, &j.fetched);
     if (e == cudaSuccess) e = cudaEventRecord(j.fetched, s->copy);
     if (e != cudaSuccess) return sloth::cuda_status(e);
     j.state = sloth::JOB_FETCHING;
@@ -864,7 +869,7 @@ int sloth_server_release(SlothServer* srv, int job_id) {
     if (j.state == sloth::JOB_PENDING || j.state == sloth::JOB_ADMITTED || j.state == sloth::JOB_FETCHING)
         return SLOTH_ERR_BUSY;
     if (j.state == sloth::JOB_DONE) sloth::free_job_memory(s, j);
-    sloth::destroy_events(j);
+    sloth::give_events(s, j);
     s->jobs.erase(it);
     return SLOTH_OK;
 }
