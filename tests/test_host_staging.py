@@ -80,42 +80,48 @@ def test_pack_grid_takes_a_snapshot_of_pinned_densities(with_range):
     assert torch.equal(g.data, ref)
 
 
-class _Pieces:
-    """The distinct pinned blocks that were asked for."""
-
-    def __init__(self, monkeypatch):
-        self.at, make = set(), runtime._pinned
-
-        def pinned(shape, dtype):
-            t = make(shape, dtype)
-            self.at.add(t.data_ptr())
-            return t
-        monkeypatch.setattr(runtime, "_pinned", pinned)
-
-
 @pytest.mark.gpu
 def test_a_host_ahead_of_its_stream_pins_no_more_pieces(monkeypatch):
-    pieces = _Pieces(monkeypatch)
+    """While the stream has not come to the first copy, no more than the pieces in flight are taken."""
+    make, late = runtime._pinned, []
     src = torch.rand(12 * STAGE + 5)
     dst = torch.empty(src.numel(), device="cuda")
-    _busy()
+    src[:100].pin_memory()                                      # the allocator is there
+    _busy(100.0)
+    before = torch.cuda.Event()
+    before.record()
+
+    def pinned(shape, dtype):
+        late.append(not before.query())
+        return make(shape, dtype)
+    monkeypatch.setattr(runtime, "_pinned", pinned)
     runtime.upload(src, dst)
     assert torch.equal(dst.cpu(), src)
-    assert len(pieces.at) <= runtime._STAGE_PIECES
+    assert len(late) == 13 and 1 <= sum(late) <= runtime._STAGE_PIECES
 
 
 @pytest.mark.gpu
 def test_a_chunked_trace_of_pageable_rays_pins_no_more_pieces(monkeypatch):
-    """Ten chunks whose uploads stand behind their lanes' traces."""
+    """Ten chunks whose uploads stand behind their lanes' traces share one set of pieces."""
     n, L = 1_500_000, 5e-3
     m = 24
     h = L / (m - 1)
     grid = runtime.pack_grid(workloads.kolmogorov_box(m, L=L, seed=1), (-L / 2,) * 3, (h,) * 3, physics.omega_of(532e-9))
     rays = workloads.gaussian_beam(n, waist=2e-3, L=L, seed=2).double().numpy()      # rows of 1.2 MB per chunk
     sched = runtime.schedule_times([L], (h,) * 3)
-    pieces = _Pieces(monkeypatch)
+    made, flying = [], []
+
+    class Staging(runtime._Staging):
+        def __init__(self):
+            super().__init__()
+            made.append(self)
+
+        def used(self, stream):
+            super().used(stream)
+            flying.append(self._open + sum(k for _, k in self._marks))
+    monkeypatch.setattr(runtime, "_Staging", Staging)
     got, steps, _ = runtime.trace_to_host(grid, rays, sched, want={"jones": "all", "steps": "all"}, chunk_rays=150_000)
-    assert len(pieces.at) <= runtime._STAGE_PIECES
+    assert len(made) == 1 and len(flying) == 60 and max(flying) <= runtime._STAGE_PIECES
     whole = runtime.trace(grid, torch.from_numpy(rays).float().cuda(), sched)
     assert torch.equal(torch.from_numpy(got["jones"]), whole["jones"].cpu()) and steps == int(whole["total_steps"])
 
