@@ -226,8 +226,7 @@ struct ServerImpl {
     TraceArgs* h_table = nullptr;   // pinned staging of the table rows
     std::vector<int> free_slots;
     std::vector<cudaEvent_t> spare_events; // of jobs that have gone, for the next ones
-    std::vector<cudaEvent_t> slot_ready;   // per slot: end of its job's admission (made at create: making
-                                           // events during a step blocked it for 8 ms now and then)
+    std::vector<cudaEvent_t> slot_ready;   // per slot: end of its job's admission
     std::unordered_map<uint64_t, GridEntry> grids;
     std::unordered_map<int, Job> jobs;
     std::deque<int> pending;
@@ -536,7 +535,8 @@ static std::deque<int>::iterator next_pending(ServerImpl* s) {
     auto it = s->pending.begin();
     for (int k = 0; k < kLook && it != s->pending.end(); ++k, ++it) {
         Job& j = s->jobs[*it];
-        j.arrived = j.arrived || !j.after || cudaEventQuery(j.after) == cudaSuccess;
+        // an error of the device counts as arrived: the admission then reports it
+        j.arrived = j.arrived || !j.after || cudaEventQuery(j.after) != cudaErrorNotReady;
         if (j.arrived) return it;
     }
     cudaGetLastError();   // cudaErrorNotReady from the queries
